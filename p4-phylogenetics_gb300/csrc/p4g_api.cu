@@ -2176,6 +2176,7 @@ static int finishLogLike(Tree *t, bool siteLikes, double *lnL)
     const int status = *treeStatusHost(t);
     if (status) {
         *treeStatusHost(t) = 0;
+        dv.cacheValid = false;   // the values that failed are not computed: the next setPrams tries them again
         return setError(P4G_ENUMERIC, "setPrams: %s did not converge",
                         (status & 1) ? "discrete gamma" : "eigensystem");
     }

@@ -1,0 +1,47 @@
+"""Model values whose rates or eigensystem cannot be formed are refused at
+every evaluation, not at the first alone, and leave nothing behind: the tree
+then evaluates good values as one that never saw the others.  An R matrix of
+zeros has no normalised Q; the incomplete gamma's series for a shape of 1e12
+is cut off after 200,000 terms."""
+import numpy
+import pytest
+
+from p4gpu import P4Error, pf, sim
+from p4gpu.engine import Engine
+
+pytestmark = pytest.mark.gpu
+
+
+def _engine(data="dna", shared=None, seed=5):
+    rng = numpy.random.default_rng(seed)
+    t = sim.yule_tree(6, rng)
+    return Engine(sim.Problem(t, [sim.make_part(t, rng, data, 40)], "failed"), shared=shared)
+
+
+def _spoil(e, what):
+    if what == "shape":
+        e.setGamma(0, 0, 1e12)
+    else:
+        sp = e.problem.parts[0]
+        e.setRMatrix(0, 0, numpy.zeros(sp.dim * (sp.dim - 1) // 2))
+
+
+def _repair(e):
+    sp = e.problem.parts[0]
+    e.setGamma(0, 0, sp.gammaShapes[0])
+    e.setRMatrix(0, 0, sim.upper_of(sp.rmats[0]))
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("data,what", [("dna", "shape"), ("dna", "matrix"), ("protein", "matrix")])
+def test_refused_every_time(data, what, precision, lib):
+    e = _engine(data)
+    pf.setPrecision(e.cTree, precision)
+    good = e.calcLogLike()
+    _spoil(e, what)
+    for _ in range(3):
+        with pytest.raises(P4Error, match="did not converge"):
+            e.calcLogLike()
+    _repair(e)
+    assert e.calcLogLike() == good
+    e.free()
