@@ -2026,7 +2026,8 @@ static int enqueueLogLike(Tree *t, bool siteLikes)
     RET(enqueuePruning(t, siteLikes));
     if (siteLikes)
         for (int p = 0; p < t->nParts; p++)
-            RET(launchSiteLikes(t->data->parts[p], t->dev.dLnl.as<double>() + t->dev.oPat[p], g_ctx.stream));
+            RET(launchSiteLikes(t->data->parts[p], t->dev.dLnl.as<double>() + t->dev.oPat[p],
+                                (const double *)t->dev.hOutDev, t->nParts, treeStatus(t), g_ctx.stream));
     return P4G_OK;
 }
 

@@ -59,7 +59,7 @@ struct Part {
     std::vector<int> seqPosIdx;        // nChar
     std::vector<int> invVec;           // nPatterns
     std::vector<int> invArr;           // dim*nPatterns
-    PinnedBuf hSiteLikes;              // nChar, written by the kernels of a getSiteLikes evaluation
+    PinnedBuf hSiteLikes;              // nChar, of the last getSiteLikes evaluation that did not fail
     bool siteLikesMade = false;        // such an evaluation has finished
     int nPatterns = 0;
     bool patternsMade = false, invarMade = false;
@@ -410,8 +410,9 @@ int pruneShapeValid(int dim, int nCat, int shape);
 int pruneKernelExists(int dim, int nCat, int shape);
 // cherryBlocks: cherry-list length (or capacity) x the largest nCat of the parts with tables
 int launchCherry(const PruneJob *dJobs, int nJobs, long long cherryBlocks, cudaStream_t s);
-// p4g_sites.cu: the part's site likelihoods from its patterns' lnL
-int launchSiteLikes(Part *p, const double *dLnl, cudaStream_t s);
+// p4g_sites.cu: the part's site likelihoods from its patterns' lnL, kept as
+// they are if the evaluation (its nParts lnLs and status, device addresses) failed
+int launchSiteLikes(Part *p, const double *dLnl, const double *partLnl, int nParts, const int *status, cudaStream_t s);
 // p4g_prune4.cu (4 states)
 int prune4NumShapes();
 int prune4ShapeValid(int nCat, int shape);

@@ -7,6 +7,11 @@
 // memory (3.2 MB for 400,000 sites).  Copying the patterns' lnL and expanding
 // them on one host core took 1.3 ms of a 1.6 ms evaluation of 61 taxa x
 // 400,000 sites.
+//
+// The buffer holds the part's last accepted evaluation: the kernel writes
+// nothing when setPrams failed or a part's lnL is not a number, the tests
+// after which the host refuses the evaluation.  Those words lie in host
+// memory; their loads are under way while the first site is exponentiated.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include "p4g_internal.h"
@@ -21,11 +26,24 @@ namespace p4g {
 
 namespace {
 
-__global__ void k_siteLikes(const double *__restrict__ lnl, const int *__restrict__ seqPos, int nChar,
-                            double *__restrict__ out)
+// partLnl, status: the evaluation's nParts lnLs and setPrams status
+__global__ void __launch_bounds__(1024) k_siteLikes(const double *__restrict__ lnl, const int *__restrict__ seqPos, int nChar,
+                            double *__restrict__ out, const volatile double *partLnl, int nParts,
+                            const volatile int *status)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nChar; i += gridDim.x * blockDim.x)
-        out[i] = exp(lnl[seqPos[i]]);
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    int good = threadIdx.x > 0 || *status == 0;
+    for (int p = threadIdx.x; p < nParts; p += blockDim.x) {
+        const double x = partLnl[p];
+        good &= x == x;
+    }
+    double v = i < nChar ? exp(lnl[seqPos[i]]) : 0.0;
+    if (!__syncthreads_and(good)) return;
+    while (i < nChar) {
+        out[i] = v;
+        i += gridDim.x * blockDim.x;
+        if (i < nChar) v = exp(lnl[seqPos[i]]);
+    }
 }
 
 }  // namespace
@@ -39,15 +57,19 @@ int Part::uploadSites(cudaStream_t s)
     return P4G_OK;
 }
 
-int launchSiteLikes(Part *p, const double *dLnl, cudaStream_t s)
+int launchSiteLikes(Part *p, const double *dLnl, const double *partLnl, int nParts, const int *status, cudaStream_t s)
 {
     RET(p->uploadSites(s));
     RET(p->hSiteLikes.ensure(sizeof(double) * std::max(p->nChar, 1)));
     void *out = nullptr;
     RET(p->hSiteLikes.device(&out));
     if (p->nChar <= 0) return P4G_OK;
-    k_siteLikes<<<std::min((p->nChar + 255) / 256, 8 * ctx().nSM), 256, 0, s>>>(dLnl, p->dSeqPos.as<int>(), p->nChar,
-                                                                              (double *)out);
+    // at most a block per SM, since every block loads the words in host memory:
+    // 400,000 sites took 433 us an evaluation with eight blocks of 256 threads
+    // per SM, 411 with one of 1,024, 409 without the test
+    const int nSM = ctx().nSM, threads = p->nChar > 256 * nSM ? 1024 : 256;
+    k_siteLikes<<<std::min((p->nChar + threads - 1) / threads, nSM), threads, 0, s>>>(
+        dLnl, p->dSeqPos.as<int>(), p->nChar, (double *)out, partLnl, nParts, status);
     P4G_CUDA(cudaGetLastError());
     return P4G_OK;
 }

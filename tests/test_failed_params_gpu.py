@@ -45,3 +45,23 @@ def test_refused_every_time(data, what, precision, lib):
     _repair(e)
     assert e.calcLogLike() == good
     e.free()
+
+
+@pytest.mark.parametrize("what", ["shape", "matrix"])
+def test_failed_evaluation_keeps_the_site_likelihoods(what, lib):
+    e = _engine()
+    e.setPrams()
+    e.logLike(1)
+    want = pf.getSiteLikes(e.cParts[0], 40)
+    _spoil(e, what)
+    for _ in range(2):
+        e.setPrams()
+        with pytest.raises(P4Error, match="did not converge"):
+            e.logLike(1)
+        assert numpy.array_equal(pf.getSiteLikes(e.cParts[0], 40), want)
+    _repair(e)
+    e.setBrLens(e.problem.tree.brLen * 1.5)
+    e.setPrams()
+    e.logLike(1)
+    assert (pf.getSiteLikes(e.cParts[0], 40) != want).any()
+    e.free()
