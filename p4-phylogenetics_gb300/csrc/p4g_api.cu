@@ -2366,6 +2366,7 @@ extern "C" int p4g_copyBigPDecks(p4g_tree *a, p4g_tree *b, int doAll)
     if (!ta || !tb) return setError(P4G_EINVAL, "copyBigPDecks: null tree");
     RET(allocTreeDev(tb));
     RET(copyDev(tb->dev.dDecks32, ta->dev.dDecks32));
+    if (ta->dev.dTcB.ptr) RET(copyDev(tb->dev.dTcB, ta->dev.dTcB));   // the tensor-core kernel's images of them
     RET(copyDev(tb->dev.dDecks64, ta->dev.dDecks64));
     RET(copyDev(tb->dev.dEqTab, ta->dev.dEqTab));
     RET(copyDev(tb->dev.dEig, ta->dev.dEig));
