@@ -2364,6 +2364,7 @@ extern "C" int p4g_copyBigPDecks(p4g_tree *a, p4g_tree *b, int doAll)
     (void)doAll;
     Tree *ta = T_(a), *tb = T_(b);
     if (!ta || !tb) return setError(P4G_EINVAL, "copyBigPDecks: null tree");
+    if (!tb->dev.haveParams && ta->dev.haveParams) RET(enqueueSetPrams(tb, -1));   // its image: rootComp and the rest
     RET(allocTreeDev(tb));
     RET(copyDev(tb->dev.dDecks32, ta->dev.dDecks32));
     if (ta->dev.dTcB.ptr) RET(copyDev(tb->dev.dTcB, ta->dev.dTcB));   // the tensor-core kernel's images of them

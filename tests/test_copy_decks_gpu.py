@@ -6,7 +6,7 @@ lnL, the FP32 pruning's; the trees' own lnLs are far further apart."""
 import numpy
 import pytest
 
-from p4gpu import pf, sim
+from p4gpu import P4Error, pf, sim
 from p4gpu.engine import Engine
 
 pytestmark = pytest.mark.gpu
@@ -32,5 +32,25 @@ def test_the_copy_takes_every_form_of_the_decks(data, shape, lib):
     pf.p4_copyBigPDecks(a.cTree, b.cTree, 1)
     assert abs(b.logLike() - want) <= 1e-6 * abs(want)
     assert abs(b.calcLogLike() - own) <= 1e-6 * abs(own)    # and its own again with its own setPrams
+    b.free()
+    a.free()
+
+
+@pytest.mark.parametrize("data", ["dna", "protein"])
+def test_into_a_tree_that_never_set_its_parameters(data, lib):
+    a, b = _pair(data)
+    want = a.calcLogLike()
+    pf.p4_copyBigPDecks(a.cTree, b.cTree, 1)
+    assert abs(b.logLike() - want) <= 1e-6 * abs(want)
+    b.free()
+    a.free()
+
+
+def test_from_a_tree_without_parameters_is_refused(lib):
+    a, b = _pair("dna")
+    with pytest.raises(P4Error):
+        pf.p4_copyBigPDecks(a.cTree, b.cTree, 1)
+    with pytest.raises(P4Error):
+        b.logLike()
     b.free()
     a.free()
