@@ -2235,8 +2235,14 @@ extern "C" int p4g_treeLogLikeBatch(p4g_tree **trees, int nTrees, int doSetPrams
         RET(enqueueLogLike(t, false));
     }
     P4G_CUDA(cudaStreamSynchronize(g_ctx.stream));
-    for (int i = 0; i < nTrees; i++) RET(finishLogLike(T_(trees[i]), false, &lnL[i]));
-    return P4G_OK;
+    // every tree's, also beside one that failed (its status is taken with it);
+    // from the last, so that the first failure's code and text remain
+    int rc = P4G_OK;
+    for (int i = nTrees - 1; i >= 0; i--) {
+        const int r = finishLogLike(T_(trees[i]), false, &lnL[i]);
+        if (r != P4G_OK) rc = r;
+    }
+    return rc;
 }
 
 extern "C" int p4g_setBrLens(p4g_tree *tt, const double *brLens)

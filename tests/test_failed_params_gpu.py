@@ -65,3 +65,18 @@ def test_failed_evaluation_keeps_the_site_likelihoods(what, lib):
     e.logLike(1)
     assert (pf.getSiteLikes(e.cParts[0], 40) != want).any()
     e.free()
+
+
+def test_every_failure_of_a_batch_call_is_taken(lib):
+    a = _engine()
+    b = _engine(shared=(a.cData, a.cParts))
+    good = [e.calcLogLike() for e in (a, b)]
+    for e in (a, b):
+        _spoil(e, "matrix")
+    with pytest.raises(P4Error, match="did not converge"):
+        pf.treeLogLikeBatch([a.cTree, b.cTree])
+    for e in (a, b):
+        _repair(e)
+    assert [e.calcLogLike() for e in (a, b)] == good
+    b.free()
+    a.free()
