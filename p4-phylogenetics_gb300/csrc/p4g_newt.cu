@@ -53,7 +53,7 @@ namespace {
 
 constexpr int kMaxDim = 20;
 constexpr int kMaxCat = 16;
-constexpr int kMaxSibs = 16;
+constexpr int kMaxSibs = 16;    // of a branch whose cl2 is formed; a node has at most one child more
 constexpr int kChunk = 64;      // patterns a block takes at a time
 constexpr int kThreads = 256;   // 4 categories of a chunk
 constexpr int kBlock = kThreads + 32;   // and a warp for the exponentials
@@ -85,7 +85,7 @@ struct NodeRef {
 struct NewtStep {
     NodeRef self;
     int isCl2, parent, parentIsRoot, nRefs;
-    NodeRef refs[kMaxSibs];
+    NodeRef refs[kMaxSibs + 1];
 };
 
 // The same with room for a binary tree's refs.
@@ -575,7 +575,7 @@ int stepOf(const Newt &N, int v, bool isCl2, NewtStep &S)
     S.parentIsRoot = (par == t->root);
     for (int c = t->nodes[isCl2 ? par : v]->leftChild; c >= 0; c = t->nodes[c]->sibling) {
         if (isCl2 && c == v) continue;
-        if (S.nRefs == kMaxSibs) return setError(P4G_EUNSUPPORTED, "newtAround: more than %d siblings", kMaxSibs);
+        if (S.nRefs == (isCl2 ? kMaxSibs : kMaxSibs + 1)) return setError(P4G_EUNSUPPORTED, "newtAround: more than %d siblings", kMaxSibs);
         S.refs[S.nRefs++] = refOf(N, c);
     }
     return P4G_OK;
