@@ -321,7 +321,9 @@ int p4g_batchLogLike(p4g_batch *b, double *lnL);
  * reports the shape and tile (patterns per block) chosen for pruning group
  * `group` of a tree (groups = distinct (dim, nCat) pairs in part order);
  * p4g_setPruneShape fixes it (after the tree's first evaluation), returning
- * P4G_EINVAL for a shape that does not apply to the group's (dim, nCat).
+ * P4G_EINVAL for a shape that does not apply to the group's (dim, nCat).  On
+ * a 4-state tree too large for the shape's P decks in shared memory the shape
+ * with the smallest footprint runs instead, and p4g_getPruneShape reports it.
  * Every shape computes the same per-pattern values. */
 int p4g_setAutotune(int on);
 /* Programmatic dependent launch of the P-deck and CUDA-core pruning kernels

@@ -1331,17 +1331,10 @@ static int refreshProgram(Tree *t)
         g.smem = pruneSmemBytes(g.dim, g.nCat, dv.nProg, t->nNodes, t->data->nTax, dv.nSlots, g.shape,
                                 dv.nClade, dv.nDeck, dv.nRow);
         if (g.smem > 227 * 1024) {   // a large tree: the tile shape with the smallest footprint
-            int best = -1, bestSmem = 0;
-            for (int sh = 0; sh < pruneNumShapes(g.dim); sh++) {
-                if (!pruneShapeValid(g.dim, g.nCat, sh)) continue;
-                const int sm = pruneSmemBytes(g.dim, g.nCat, dv.nProg, t->nNodes, t->data->nTax, dv.nSlots, sh,
-                                              dv.nClade, dv.nDeck, dv.nRow);
-                if (sm <= 227 * 1024 && (best < 0 || sm < bestSmem)) {
-                    best = sh;
-                    bestSmem = sm;
-                }
-            }
-            if (best < 0)
+            int bestSmem = 0;
+            const int best = pruneShapeSmallest(g.dim, g.nCat, dv.nProg, t->nNodes, t->data->nTax, dv.nSlots, dv.nClade,
+                                                dv.nDeck, dv.nRow, &bestSmem);
+            if (bestSmem > PRUNE_SMEM_MAX)
                 return setError(P4G_EUNSUPPORTED,
                                 "tree too large for the fused kernel's shared memory (%d bytes)", g.smem);
             g.shape = best;
@@ -1709,9 +1702,13 @@ static int autotune(Tree *t, bool fresh = false)
         gr.shape = bestShape;
         g_tuneCache[key] = bestShape;
     }
-    for (auto &gr : dv.groups)
+    for (auto &gr : dv.groups) {
         gr.smem = pruneSmemBytes(gr.dim, gr.nCat, dv.nProg, t->nNodes, t->data->nTax, dv.nSlots, gr.shape,
                                  dv.nClade, dv.nDeck, dv.nRow);
+        if (gr.smem > PRUNE_SMEM_MAX)   // no timed shape fits, or one kept for a smaller program does not
+            gr.shape = pruneShapeSmallest(gr.dim, gr.nCat, dv.nProg, t->nNodes, t->data->nTax, dv.nSlots, dv.nClade,
+                                          dv.nDeck, dv.nRow, &gr.smem);
+    }
     RET(waitImage(t));
     RET(layoutBlocks(t));
     RET(uploadImage(t));
@@ -1904,11 +1901,12 @@ extern "C" int p4g_setPruneShape(p4g_tree *tt, int group, int shape)
                         gr.nCat);
     RET(waitImage(t));
     if (dv.progDirty) RET(refreshProgram(t));
-    const int smem = pruneSmemBytes(gr.dim, gr.nCat, dv.nProg, t->nNodes, t->data->nTax, dv.nSlots, shape, dv.nClade,
-                                    dv.nDeck, dv.nRow);
-    if (smem > 227 * 1024)
+    int smem = 0;
+    const int runs = pruneShapeFor(gr.dim, gr.nCat, dv.nProg, t->nNodes, t->data->nTax, dv.nSlots, shape, dv.nClade,
+                                   dv.nDeck, dv.nRow, &smem);
+    if (smem > PRUNE_SMEM_MAX)
         return setError(P4G_EUNSUPPORTED, "setPruneShape: shape %d needs %d bytes of shared memory", shape, smem);
-    gr.shape = shape;
+    gr.shape = runs;
     gr.smem = smem;
     RET(layoutBlocks(t));
     RET(uploadImage(t));

@@ -259,7 +259,11 @@ int cladeBuild(Tree *t, const std::vector<int> &need, const std::vector<int> &cl
         int shape = defaultShape(keys[gi].first);
         if (keys[gi].first == 4) shape = keys[gi].second % 2 == 0 ? 8 : 3;
         auto it = dv.cladeShape.find(keys[gi].first * 64 + keys[gi].second);   // chosen by the timing
-        if (it != dv.cladeShape.end()) shape = it->second;
+        if (it != dv.cladeShape.end()) {
+            int bytes = 0;
+            shape = pruneShapeFor(keys[gi].first, keys[gi].second, *std::max_element(progLen.begin(), progLen.end()), nn,
+                                  L, *std::max_element(slots.begin(), slots.end()), it->second, 0, -1, -1, &bytes);
+        }
         shapeOfGroup[gi] = shape;
         tileOfGroup[gi] = pruneTile(keys[gi].first, keys[gi].second, shape);
     }

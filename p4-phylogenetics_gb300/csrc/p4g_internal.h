@@ -418,7 +418,9 @@ int prune4NumShapes();
 int prune4ShapeValid(int nCat, int shape);
 int prune4KernelExists(int nCat, int shape);
 int prune4Tile(int nCat, int shape);
+int prune4Smallest(int nCat);
 int prune4SmemBytes(int nCat, int nProg, int nDecks, int nRows, int nSlots, int shape, int nClade);
+int prune4FirstBytes(int nCat, int nProg, int nDecks, int nRows, int nSlots, int shape, int nClade);
 int launchPrune4(const PruneJob *dJobs, const BlockDesc *dBlocks, int nTiles, int nCat, int smemBytes, int shape,
                  cudaStream_t s, const int *nTilesDev, int early);
 // p4g_prune_tc.cu
@@ -427,6 +429,14 @@ int launchPruneTc(const PruneJob *dJobs, const BlockDesc *dBlocks, int nTiles, i
                   const int *nTilesDev = nullptr, int early = 0);
 int pruneSmemBytes(int dim, int nCat, int nProg, int nNodes, int nTax, int nSlots, int shape, int nClade = 0,
                    int nDeck = -1, int nRow = -1);
+constexpr int PRUNE_SMEM_MAX = 227 * 1024;
+// The shape that runs where `shape` is asked for (bytes: its shared memory,
+// above PRUNE_SMEM_MAX when none fits).
+int pruneShapeFor(int dim, int nCat, int nProg, int nNodes, int nTax, int nSlots, int shape, int nClade, int nDeck,
+                  int nRow, int *bytes);
+// The shape with the smallest footprint (bytes as above).
+int pruneShapeSmallest(int dim, int nCat, int nProg, int nNodes, int nTax, int nSlots, int nClade, int nDeck, int nRow,
+                       int *bytes);
 
 // host math shared with device code (p4g_math.cuh)
 int discreteGammaHost(double alpha, int K, double *rates);

@@ -801,6 +801,33 @@ int pruneSmemBytes(int dim, int nCat, int nProg, int nNodes, int nTax, int nSlot
     return smemLayout(nProg, decks, rows, dim, nCat, s.tp, s.ppt, s.g, nSlots, s.sdeck, nClade).total;
 }
 
+int pruneShapeSmallest(int dim, int nCat, int nProg, int nNodes, int nTax, int nSlots, int nClade, int nDeck, int nRow,
+                       int *bytes)
+{
+    int best = dim == 4 ? prune4Smallest(nCat) : 0;
+    *bytes = pruneSmemBytes(dim, nCat, nProg, nNodes, nTax, nSlots, best, nClade, nDeck, nRow);
+    for (int sh = 0; sh < pruneNumShapes(dim); sh++) {
+        if (!pruneShapeValid(dim, nCat, sh)) continue;
+        const int sm = pruneSmemBytes(dim, nCat, nProg, nNodes, nTax, nSlots, sh, nClade, nDeck, nRow);
+        if (sm < *bytes) {
+            best = sh;
+            *bytes = sm;
+        }
+    }
+    return best;
+}
+
+int pruneShapeFor(int dim, int nCat, int nProg, int nNodes, int nTax, int nSlots, int shape, int nClade, int nDeck,
+                  int nRow, int *bytes)
+{
+    *bytes = pruneSmemBytes(dim, nCat, nProg, nNodes, nTax, nSlots, shape, nClade, nDeck, nRow);
+    const int decks = nDeck >= 0 ? nDeck : nNodes, rows = nRow >= 0 ? nRow : nTax;
+    if (*bytes <= PRUNE_SMEM_MAX || dim != 4 ||
+        prune4FirstBytes(nCat, nProg, decks, rows, nSlots, shape, nClade) > PRUNE_SMEM_MAX)
+        return shape;
+    return pruneShapeSmallest(dim, nCat, nProg, nNodes, nTax, nSlots, nClade, nDeck, nRow, bytes);
+}
+
 template <int DIM, int NC, int TP, int PPT, bool SDECK, int G>
 static int launchT(const PruneJob *dJobs, const BlockDesc *dBlocks, int nTiles, int smemBytes,
                    cudaStream_t s, const int *nTilesDev, int early)

@@ -29,6 +29,7 @@
 //     usual rescale is one product.
 // An odd category count repeats its last category in the pair's upper half.
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <algorithm>
 #include "p4g_internal.h"
 #include "p4g_prune_common.cuh"
@@ -713,7 +714,8 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
 // are what large alignments wait for), P decks staged in shared memory (else
 // read through L1, which leaves shared memory to the codes and the stack),
 // lanes per pattern (the category pairs spread over 2 lanes, for alignments
-// of few patterns; counts whose pairs do not divide take one lane), resident
+// of few patterns; counts whose pairs do not divide take one lane and half the
+// threads, so that the tile stays tp / g * ppt patterns), resident
 // blocks the registers are held to, and the category counts the shape is
 // offered for (a divisor, or 3 and 4 alone).
 struct Shape4 {
@@ -722,28 +724,48 @@ struct Shape4 {
     int g, mb, div;
     bool only34;
 };
-// every tile holds 64 to 512 patterns
+// every tile holds 64 to 512 patterns; the last shape, for odd counts, is not
+// timed, but the smallest in shared memory, as shape 8 is for even ones
 constexpr Shape4 kShapes4[] = {{128, 1, true, 1, 0, 1, false},  {128, 2, true, 1, 0, 1, false},
                                {256, 1, true, 1, 0, 1, false},  {256, 1, false, 1, 0, 1, false},
                                {128, 2, false, 1, 0, 1, false}, {512, 1, false, 1, 0, 1, false},
                                {128, 1, true, 2, 0, 4, false},  {256, 1, false, 2, 0, 2, false},
                                {128, 1, false, 2, 0, 2, false}, {256, 2, true, 2, 0, 4, false},
                                {128, 2, true, 2, 0, 4, false},  {128, 4, true, 2, 0, 1, true},
-                               {128, 2, true, 1, 4, 1, true}};
-constexpr int kNumShapes4 = 13;
+                               {128, 2, true, 1, 4, 1, true},
+                               {128, 1, false, 1, 0, 1, false}};
+constexpr int kNumShapes4 = 13;   // timed
+constexpr int kSmallOdd4 = 13, kSmallEven4 = 8;
+
+// Where a caller may ask for a shape: (threads, tile, decks staged) as the
+// numbers were first given out, 16 floats a deck and category.  The forms above
+// hold more for some of them (decks in category pairs, decks staged where they
+// were not, larger tiles); a tree that the first form fits and today's does not
+// runs the smallest shape.  (Refused instead, shapes 6 and 10 were lost from 500
+// taxa on and a tree of 800 taxa and one category could not be evaluated.)
+struct First4 {
+    int tp, tile;
+    bool sdeck;
+};
+constexpr First4 kFirst4[kNumShapes4] = {{128, 128, true},  {128, 256, true},  {256, 256, true}, {256, 256, false},
+                                         {128, 256, false}, {512, 512, false}, {256, 64, false}, {256, 128, false},
+                                         {128, 64, false},  {256, 64, true},   {512, 128, false}, {256, 256, true},
+                                         {128, 256, true}};
 
 constexpr int lanes4(int nCat, int shape)
 {
     const int g = kShapes4[shape].g, pairs = (nCat + 1) / 2;
     return (nCat % 2 == 0 && pairs % g == 0) ? g : 1;
 }
+constexpr int threads4(int nCat, int shape) { return kShapes4[shape].tp / kShapes4[shape].g * lanes4(nCat, shape); }
 
 template <int NC, int SH>
 int launchShape4(const PruneJob *dJobs, const BlockDesc *dBlocks, int nTiles, int smemBytes, cudaStream_t s,
                  const int *nTilesDev, int early)
 {
     constexpr Shape4 S = kShapes4[SH];
-    auto k = k_prune4<NC, S.tp, S.ppt, S.sdeck, lanes4(NC, SH), S.mb>;
+    constexpr int TP = threads4(NC, SH);
+    auto k = k_prune4<NC, TP, S.ppt, S.sdeck, lanes4(NC, SH), S.mb>;
     static int configured = 0;
     static int perSM = 0, perSMsmem = -1;
     if (smemBytes > 48 * 1024 && configured < smemBytes) {
@@ -751,12 +773,12 @@ int launchShape4(const PruneJob *dJobs, const BlockDesc *dBlocks, int nTiles, in
         configured = smemBytes;
     }
     if (perSMsmem != smemBytes) {
-        P4G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k, S.tp, smemBytes));
+        P4G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k, TP, smemBytes));
         perSMsmem = smemBytes;
     }
     if (perSM < 1) return setError(P4G_EUNSUPPORTED, "pruning kernel does not fit on an SM (%d B smem)", smemBytes);
     const int grid = std::min(nTiles, perSM * ctx().nSM);
-    P4G_CUDA(launchPdl(k, dim3(grid), dim3(S.tp), smemBytes, s, dJobs, dBlocks, nTiles, nTilesDev, early));
+    P4G_CUDA(launchPdl(k, dim3(grid), dim3(TP), smemBytes, s, dJobs, dBlocks, nTiles, nTilesDev, early));
     return P4G_OK;
 }
 
@@ -775,6 +797,7 @@ int launchCat4(const PruneJob *dJobs, const BlockDesc *dBlocks, int nTiles, int 
     case 10: if constexpr (NC % 4 == 0) return launchShape4<NC, 10>(dJobs, dBlocks, nTiles, smemBytes, s, nTilesDev, early); break;
     case 11: if constexpr (NC == 3 || NC == 4) return launchShape4<NC, 11>(dJobs, dBlocks, nTiles, smemBytes, s, nTilesDev, early); break;
     case 12: if constexpr (NC == 3 || NC == 4) return launchShape4<NC, 12>(dJobs, dBlocks, nTiles, smemBytes, s, nTilesDev, early); break;
+    case kSmallOdd4: if constexpr (NC % 2 == 1) return launchShape4<NC, kSmallOdd4>(dJobs, dBlocks, nTiles, smemBytes, s, nTilesDev, early); break;
 #undef P4G_SH
     default: break;
     }
@@ -787,6 +810,7 @@ int prune4NumShapes() { return kNumShapes4; }
 
 int prune4ShapeValid(int nCat, int shape)
 {
+    if (shape == kSmallOdd4) return nCat % 2;
     if (shape < 0 || shape >= kNumShapes4) return 0;
     if (kShapes4[shape].only34) return nCat == 3 || nCat == 4;
     return nCat % kShapes4[shape].div == 0;
@@ -797,12 +821,20 @@ int prune4KernelExists(int nCat, int shape)
     return prune4ShapeValid(nCat, shape) && ((nCat >= 1 && nCat <= 6) || nCat == 8);
 }
 
-int prune4Tile(int nCat, int shape) { return kShapes4[shape].tp / lanes4(nCat, shape) * kShapes4[shape].ppt; }
+int prune4Tile(int nCat, int shape) { return threads4(nCat, shape) / lanes4(nCat, shape) * kShapes4[shape].ppt; }
+int prune4Smallest(int nCat) { return nCat % 2 ? kSmallOdd4 : kSmallEven4; }
 
 int prune4SmemBytes(int nCat, int nProg, int nDecks, int nRows, int nSlots, int shape, int nClade)
 {
     const Shape4 &S = kShapes4[shape];
-    return layout4(nProg, nDecks, nRows, nCat, S.tp, prune4Tile(nCat, shape), nSlots, S.sdeck, nClade).total;
+    return layout4(nProg, nDecks, nRows, nCat, threads4(nCat, shape), prune4Tile(nCat, shape), nSlots, S.sdeck, nClade).total;
+}
+
+int prune4FirstBytes(int nCat, int nProg, int nDecks, int nRows, int nSlots, int shape, int nClade)
+{
+    if (shape >= kNumShapes4) return INT_MAX;
+    const First4 &F = kFirst4[shape];
+    return layout4(nProg, 0, nRows, nCat, F.tp, F.tile, nSlots, false, nClade).total + (F.sdeck ? nDecks * nCat * 64 : 0);
 }
 
 int launchPrune4(const PruneJob *dJobs, const BlockDesc *dBlocks, int nTiles, int nCat, int smemBytes, int shape,
