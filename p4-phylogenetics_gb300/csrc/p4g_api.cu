@@ -2101,7 +2101,7 @@ static int buildTable64(Tree *t)
         dv.oCl64[p] = nCl;
         nCl += (size_t)dv.nInternal64 * mp.nCat * mp.dim * dp->nPatPad;
         dv.oPartials64[p] = nPartials;
-        nPartials += (dp->nPatterns + 63) / 64;   // a block takes at least 64 patterns
+        nPartials += (dp->nPatterns + 3) / 4;   // a block takes at least 4 patterns
     }
     RET(dv.dCl64.ensure(sizeof(double) * nCl));
     RET(dv.dPartials64.ensure(sizeof(double) * nPartials));

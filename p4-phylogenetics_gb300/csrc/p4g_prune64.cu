@@ -21,6 +21,7 @@
 // need 0.6 ms.  An evaluation with a launch per node took 1.23 ms (245 us for
 // 32 taxa x 7 k patterns, all launch and tail), with this kernel 0.79 ms (106 us).
 #include <cuda_runtime.h>
+#include <algorithm>
 #include "p4g_internal.h"
 #include "p4g_prune64.cuh"
 
@@ -79,19 +80,31 @@ __device__ __forceinline__ void childFactor(const Node64Job &J, const int *node,
     }
 }
 
-// A block takes `chunk` patterns in every category; thread i of the chunk's
-// chunk * nCat pairs is (category i / chunk, pattern i % chunk).
-constexpr int kThreads64 = 256;
-inline int chunk64(int nCat) { return nCat == 1 ? 256 : nCat == 2 ? 128 : 64; }
+// A block takes `chunk` patterns in every category, one thread each: thread i is
+// (category i / chunk, pattern i % chunk).  At most 256 threads, 128 for 20
+// states, whose 255 registers a thread leave an SM one block of 256 and the last
+// of a few such blocks alone on it.  Whole warps of a category where two or more
+// fit (three categories of 84 patterns instead of 64: 105 -> 125 us for 32 taxa x
+// 20,000 DNA patterns; in blocks of 192 threads 114), else multiples of four patterns.  Chunks of 64 whatever
+// the count, in passes of 256 threads, took 2.56 ms for 48 taxa x 10,000 protein
+// patterns x 4 categories, 1.53 ms for 16 x 1,000 x 16 and 0.140 ms for 16 x 1,000
+// DNA patterns x 16; these 1.99, 0.294 and 0.069 (a launch per node: 2.18, 0.431,
+// 0.141).
+constexpr int maxThreads64(int dim) { return dim > 4 ? 128 : 256; }
+inline int chunk64(int dim, int nCat)
+{
+    const int n = maxThreads64(dim) / nCat;
+    return n >= 64 ? n / 32 * 32 : std::max(4, n / 4 * 4);
+}
+static_assert(MAX_CAT * 4 <= maxThreads64(20), "a chunk of 4 patterns is one pass");
 
 template <int DIM>
-__global__ void __launch_bounds__(kThreads64) k_prune64(const Node64Job *__restrict__ job, int chunk)
+__global__ void __launch_bounds__(maxThreads64(DIM)) k_prune64(const Node64Job *__restrict__ job, int chunk)
 {
     const Node64Job &J = *job;
     const int p0 = blockIdx.x * chunk;
-    for (int i = threadIdx.x; i < chunk * J.nCat; i += kThreads64) {
-        const int cat = i / chunk, pat = p0 + i % chunk;
-        if (pat >= J.nPat) continue;
+    const int cat = threadIdx.x / chunk, pat = p0 + threadIdx.x % chunk;
+    if (cat < J.nCat && pat < J.nPat) {
         double last[DIM];
 #pragma unroll
         for (int s = 0; s < DIM; s++) last[s] = 0.0;
@@ -122,10 +135,9 @@ __global__ void __launch_bounds__(kThreads64) k_prune64(const Node64Job *__restr
     }
     __syncthreads();
     // root reduction, one pattern a thread, (category, state) in order
-    const int pat = p0 + threadIdx.x;
     double v = 0.0;
     int bad = 0;
-    if (threadIdx.x < chunk && pat < J.nPat) {
+    if (cat == 0 && pat < J.nPat) {
         const double *root = J.cl + (size_t)J.rootInternal * J.nCat * DIM * J.nPatPad + pat;
         double like = 0.0;
         uint32_t mask = (DIM >= 32) ? 0xffffffffu : ((1u << DIM) - 1u);
@@ -156,14 +168,14 @@ __global__ void __launch_bounds__(kThreads64) k_prune64(const Node64Job *__restr
         else v = J.counts[pat] * log(like);
     }
     for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    __shared__ double red[kThreads64 / 32];
+    __shared__ double red[maxThreads64(DIM) / 32];
     __shared__ int sLast;
     const int anyBad = __syncthreads_or(bad);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
     if (threadIdx.x == 0) {
         double s = red[0];
-        for (int w = 1; w < chunk / 32; w++) s += red[w];
+        for (int w = 1; w < (chunk + 31) / 32; w++) s += red[w];
         J.partials[blockIdx.x] = s;
         if (anyBad) atomicOr(J.badFlag, 1);
         __threadfence();
@@ -185,8 +197,9 @@ __global__ void __launch_bounds__(kThreads64) k_prune64(const Node64Job *__restr
 template <int DIM>
 static int launch64(const Node64Job *dJob, const Node64Job &h, cudaStream_t s)
 {
-    const int chunk = chunk64(h.nCat);
-    k_prune64<DIM><<<(h.nPat + chunk - 1) / chunk, kThreads64, 0, s>>>(dJob, chunk);
+    const int chunk = chunk64(DIM, h.nCat);
+    const int threads = chunk >= 64 ? maxThreads64(DIM) : (chunk * h.nCat + 31) / 32 * 32;
+    k_prune64<DIM><<<(h.nPat + chunk - 1) / chunk, threads, 0, s>>>(dJob, chunk);
     P4G_CUDA(cudaGetLastError());
     return P4G_OK;
 }
