@@ -2350,7 +2350,7 @@ extern "C" int p4g_treeDeviceBytes(p4g_tree *tt, long long *treeBytes, long long
             const Part *dp = t->data->parts[p];
             if (dp)
                 db += (long long)(dp->dCodes.bytes + dp->dCounts.bytes + dp->dInvMask.bytes + dp->dEquates.bytes +
-                                  dp->dPat32.bytes + dp->dEqInt.bytes + dp->dSeqPos.bytes);
+                                  dp->dPat32.bytes + dp->dEqInt.bytes + dp->dSeqPos.bytes + dp->dUniforms.bytes);
         }
     *dataBytes = db;
     return P4G_OK;

@@ -83,6 +83,11 @@ struct Part {
     DevBuf dSeqPos;               // seqPosIdx [nChar], of the data uploaded as generation sitesGen
     unsigned long long sitesGen = 0;
     int uploadSites(cudaStream_t s);
+    // ancestral-state draws (p4g_sim.cu): the caller's uniforms and the draws,
+    // in use during a call alone, so that the data and not each of their
+    // trees hold the 24 bytes a site
+    DevBuf dUniforms;
+    PinnedBuf hDraws;
 };
 
 struct Data {
@@ -331,8 +336,6 @@ struct TreeDev {
     // products, the round's tables and counters; its results in host memory
     DevBuf dCl2, dNewtA, dNewt;
     PinnedBuf hNewt;
-    DevBuf dUniforms;   // ancestral-state draws (p4g_sim.cu): the caller's uniforms
-    PinnedBuf hDraws;   // and the draws
     std::vector<size_t> oCl64, oPartials64;
     int nInternal64 = 0;
 };

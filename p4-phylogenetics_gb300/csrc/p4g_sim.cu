@@ -252,17 +252,17 @@ extern "C" int p4g_drawAncStates(p4g_tree *tt, int pNum, const double *uniforms,
     const ModelPart &mp = t->model->parts[pNum];
     Part *dp = t->data->parts[pNum];
     const int nChar = dp->nChar;
-    // the draws land in a host buffer the tree keeps, the failure flag behind them
+    // the draws land in a host buffer the data keep, the failure flag behind them
     const size_t drawBytes = sizeof(int) * 4 * (size_t)nChar;
-    RET(dv.hDraws.ensure(drawBytes + 16));
+    RET(dp->hDraws.ensure(drawBytes + 16));
     void *hDev = nullptr;
-    RET(dv.hDraws.device(&hDev));
-    int *failed = (int *)((char *)dv.hDraws.ptr + drawBytes);
+    RET(dp->hDraws.device(&hDev));
+    int *failed = (int *)((char *)dp->hDraws.ptr + drawBytes);
     *failed = 0;
-    if (uniforms) RET(dv.dUniforms.ensure(sizeof(double) * nChar));
+    if (uniforms) RET(dp->dUniforms.ensure(sizeof(double) * nChar));
     cudaStream_t s = ctx().stream;
     RET(dp->uploadSites(s));
-    if (uniforms) P4G_CUDA(cudaMemcpyAsync(dv.dUniforms.ptr, uniforms, sizeof(double) * nChar, cudaMemcpyHostToDevice, s));
+    if (uniforms) P4G_CUDA(cudaMemcpyAsync(dp->dUniforms.ptr, uniforms, sizeof(double) * nChar, cudaMemcpyHostToDevice, s));
     const PruneJob *hj = (const PruneJob *)((const char *)dv.hImg.ptr + dv.oJobs);
     AncPart A;
     A.rootCL = dv.dRootCL.as<float>() + dv.oRootCL[pNum];
@@ -270,7 +270,7 @@ extern "C" int p4g_drawAncStates(p4g_tree *tt, int pNum, const double *uniforms,
     A.invMask = dp->dInvMask.as<uint32_t>();
     A.seqPosIdx = dp->dSeqPos.as<int>();
     A.rootComp = hj[pNum].rootComp;
-    A.uniforms = uniforms ? dv.dUniforms.as<double>() : nullptr;
+    A.uniforms = uniforms ? dp->dUniforms.as<double>() : nullptr;
     A.draws = (int *)hDev;
     A.failed = (int *)((char *)hDev + drawBytes);
     A.seed = seed;
@@ -290,7 +290,7 @@ extern "C" int p4g_drawAncStates(p4g_tree *tt, int pNum, const double *uniforms,
         P4G_CUDA(cudaGetLastError());
     }
     P4G_CUDA(cudaStreamSynchronize(s));
-    memcpy(draws, dv.hDraws.ptr, drawBytes);
+    memcpy(draws, dp->hDraws.ptr, drawBytes);
     if (*failed)
         return setError(P4G_ENUMERIC, "drawAncStates: the ancestral state picker found no state for some site");
     return P4G_OK;
