@@ -64,10 +64,11 @@ int launchSiteLikes(Part *p, const double *dLnl, const double *partLnl, int nPar
     void *out = nullptr;
     RET(p->hSiteLikes.device(&out));
     if (p->nChar <= 0) return P4G_OK;
-    // at most a block per SM, since every block loads the words in host memory:
-    // 400,000 sites took 433 us an evaluation with eight blocks of 256 threads
-    // per SM, 411 with one of 1,024, 409 without the test
-    const int nSM = ctx().nSM, threads = p->nChar > 256 * nSM ? 1024 : 256;
+    // a block per SM with an even share of the sites, since every block loads
+    // the words in host memory: 400,000 sites took 433 us an evaluation with eight
+    // blocks of 256 threads per SM, 411 with one of 1,024, 409 without the test
+    const int nSM = ctx().nSM;
+    const int threads = std::min(1024, ((p->nChar + nSM - 1) / nSM + 31) / 32 * 32);
     k_siteLikes<<<std::min((p->nChar + threads - 1) / threads, nSM), threads, 0, s>>>(
         dLnl, p->dSeqPos.as<int>(), p->nChar, (double *)out, partLnl, nParts, status);
     P4G_CUDA(cudaGetLastError());
