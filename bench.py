@@ -25,9 +25,9 @@ batched_8_trees : 8 trees of the workload (the chains of an MCMCMC), each
         one captured CUDA graph per step; host wall clock.
 mcmc  : MCMC throughput and ESS/s on the MCMC workloads (after the timed
         region; --no-mcmc skips it).
---impl reference : the reference algorithm's CPU implementation (the
-        oracle's restatement of Pf/p4_node.c + Pf/p4_tree.c, FP64), pattern-
-        parallel over all host cores, on the same workload.
+--impl reference : the reference's own C core (Pf/*.c, FP64), pattern-
+        parallel over all host cores, on the same workload; one line saying
+        why, where that core cannot be built.
 Multi-GPU (torchrun): independent replicas, one per rank; value sums ranks
 over the max-over-ranks time.
 """
@@ -171,6 +171,31 @@ def cpu_mcmcmc_parallel(config, nChains, seconds):
         ev.close()
 
 
+def reference_core():
+    """None when the reference's own C core can be used here (built, or built
+    now from its staged sources), else why not, in one line."""
+    from oracle import oracle
+    if not oracle.have_ref():
+        oracle.build(ref=True)
+    if oracle.have_ref():
+        return None
+    if not oracle.have_ref_sources():
+        return "the reference's C sources are not on this machine"
+    return "the reference's C core did not build on this machine"
+
+
+def cpu_part(measure, why):
+    """What a CPU baseline of the MCMC section measured, or that it is
+    unavailable and why: a baseline that cannot run costs its own entry alone,
+    never the measurements of the GPU."""
+    if why is None:
+        try:
+            return measure()
+        except Exception as ex:
+            why = repr(ex)
+    return {"unavailable": why}
+
+
 def mcmc_section(cpu=True):
     """MCMC throughput and ESS/s on the MCMC workloads (run after the timed
     region), each run long enough that every reported ESS reaches 100 (or a
@@ -207,17 +232,21 @@ def mcmc_section(cpu=True):
                      "sample every 10", "fp64_single_eval_ms": fp64_ms, "fp64_lnL": lnl64, "generations": gens,
          "seconds": dt, "gens_per_s": gens / dt, "acceptance": m.acceptance()}
     d.update(ess_block(m.samples, dt))
-    if cpu:
-        one, agg = cpu_chains("dna16", 1, 1500, 1)
+    why = reference_core() if cpu else None
+
+    def dna16_cpu():
+        one, _ = cpu_chains("dna16", 1, 1500, 1)
         _, aggK = cpu_chains("dna16", 1, 1500, ncpu)
-        d["cpu_baseline"] = {"kind": "reference", "gens_per_s": one, "cores": 1,
-                             "gens_per_s_k_cores": aggK, "k": ncpu,
-                             "ess_per_s": {k: d["ess_" + k] / gens * one for k in ("lnL", "treeLength", "alpha")
-                                           if "ess_" + k in d},
-                             "sample": "1,500 generations of the same sampler on the reference's own C core "
-                                       "(Pf/*.c compiled on this host), p4 part-granular updates; k cores: k "
-                                       "independent chains, aggregate; ESS/s = the GPU run's ESS per generation "
-                                       "x these generations/s"}
+        return {"kind": "reference", "gens_per_s": one, "cores": 1,
+                "gens_per_s_k_cores": aggK, "k": ncpu,
+                "ess_per_s": {k: d["ess_" + k] / gens * one for k in ("lnL", "treeLength", "alpha")
+                              if "ess_" + k in d},
+                "sample": "1,500 generations of the same sampler on the reference's own C core "
+                          "(Pf/*.c compiled on this host), p4 part-granular updates; k cores: k "
+                          "independent chains, aggregate; ESS/s = the GPU run's ESS per generation "
+                          "x these generations/s"}
+    if cpu:
+        d["cpu_baseline"] = cpu_part(dna16_cpu, why)
     out["dna16_single_chain"] = d
     prob = sim.make_config("mcmcmc32")
     note = ("8 chains (temps 0,0.1,...,0.7) x 12 partitions (8 DNA + 4 protein, 200-30,000 sites) on 32 taxa; "
@@ -247,17 +276,19 @@ def mcmc_section(cpu=True):
         else:
             d["ess_per_s_from_graph_ess_per_gen"] = {k: v * n / dt for k, v in essPerGen.items()}
         out["mcmcmc32_8chains_12parts_" + ev] = d
-    if cpu:
+
+    def mcmcmc32_cpu():
         gk, dk = cpu_mcmcmc_parallel("mcmcmc32", 8, 15.0)
         one, _ = cpu_chains("mcmcmc32", 8, 3, 1)
-        out["mcmcmc32_8chains_12parts_graph"]["cpu_baseline"] = {
-            "kind": "reference", "gens_per_s": one, "cores": 1, "gens_per_s_8_cores": gk / dk, "k": 8,
-            "ess_per_s": {k: v * one for k, v in essPerGen.items()},
-            "ess_per_s_8_cores": {k: v * gk / dk for k, v in essPerGen.items()},
-            "sample": "the same 8-chain sampler on the reference's own C core with p4's part-granular updates: "
-                      "3 generations on 1 core, and %d generations with the 8 chains' evaluations on 8 "
-                      "processes (one per core); ESS/s = the GPU graph run's ESS per generation x these "
-                      "generations/s" % gk}
+        return {"kind": "reference", "gens_per_s": one, "cores": 1, "gens_per_s_8_cores": gk / dk, "k": 8,
+                "ess_per_s": {k: v * one for k, v in essPerGen.items()},
+                "ess_per_s_8_cores": {k: v * gk / dk for k, v in essPerGen.items()},
+                "sample": "the same 8-chain sampler on the reference's own C core with p4's part-granular updates: "
+                          "3 generations on 1 core, and %d generations with the 8 chains' evaluations on 8 "
+                          "processes (one per core); ESS/s = the GPU graph run's ESS per generation x these "
+                          "generations/s" % gk}
+    if cpu:
+        out["mcmcmc32_8chains_12parts_graph"]["cpu_baseline"] = cpu_part(mcmcmc32_cpu, why)
     out["dna32het6_learned"] = learned_seeds((5, 6, 7))
     return out
 
@@ -592,6 +623,10 @@ def reference_arm(args):
     if rank != 0:
         return
     from p4gpu import sim
+    why = reference_core()
+    if why is not None:   # this arm is the reference's own code or nothing
+        print(json.dumps({"impl": "reference", "unavailable": why}))
+        return
     problem = sim.make_config(args.config)
     nProcs = len(os.sched_getaffinity(0)) if hasattr(os, "sched_getaffinity") else (os.cpu_count() or 1)
     # size the steps: one evaluation per step per process, about 1 s of work per step at most
@@ -599,7 +634,6 @@ def reference_arm(args):
     one = max(statistics.median(t[1]) for t in probe.values())
     per_step = max(1, int(1.0 / max(one, 1e-6)))
     res = run_cpu_arm(args.config, nProcs, nProcs, nEvals=(args.warmup + args.steps) * per_step)
-    kind = res[0][0]
     # step i of every process ran at the same time; the step takes as long as its slowest process
     steps = []
     for i in range(args.warmup, args.warmup + args.steps):
@@ -612,14 +646,13 @@ def reference_arm(args):
             "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": DATA,
             "impl": "reference",
             "config": workload_config(problem, args.gpus),
-            "cpu_baseline": {"value": value, "unit": "evals/s", "cores": nProcs, "kind": kind,
+            "cpu_baseline": {"value": value, "unit": "evals/s", "cores": nProcs, "kind": "reference",
                              "sample": "%d steps of %d evaluation(s) each: p4's allBrLens evaluation "
-                                       "(p4_calculateBigPDecks of every node + p4_treeLogLike) by the %s, "
+                                       "(p4_calculateBigPDecks of every node + p4_treeLogLike) by the "
+                                       "reference's own C core (Pf/*.c compiled on this host), "
                                        "the patterns split round-robin over %d processes pinned one per core; "
                                        "a step takes as long as its slowest process"
-                                       % (args.steps, per_step,
-                                          "reference's own C core (Pf/*.c compiled on this host)"
-                                          if kind == "reference" else "oracle's FP64 restatement", nProcs)},
+                                       % (args.steps, per_step, nProcs)},
             "e2e": {"value": value, "unit": "evals/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
             "lnL": lnl}
     print(json.dumps(line))
