@@ -1113,7 +1113,7 @@ static int allocTreeDev(Tree *t)
         for (int p = 0; p < nP; p++) {
             const int K = m->parts[p].dim + 1 + d->parts[p]->nPartial;
             dv.oCherryTab[p] = (size_t)-1;
-            if (m->parts[p].dim < 20) continue;   // measured: pays for 20 states, not for 4
+            if (m->parts[p].dim != CHERRY_DIM) continue;   // measured: pays for 20 states, not for 4
             // a table of K x K code pairs is built every evaluation: it pays only
             // when the part has clearly more patterns than code pairs
             if (d->parts[p]->nPatterns < 2 * K * K) continue;

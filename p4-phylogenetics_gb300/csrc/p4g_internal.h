@@ -411,6 +411,7 @@ int pruneNumShapes(int dim);
 int pruneTile(int dim, int nCat, int shape);
 int pruneShapeValid(int dim, int nCat, int shape);
 int pruneKernelExists(int dim, int nCat, int shape);
+constexpr int CHERRY_DIM = 20;   // states of the parts that have cherry tables
 // cherryBlocks: cherry-list length (or capacity) x the largest nCat of the parts with tables
 int launchCherry(const PruneJob *dJobs, int nJobs, long long cherryBlocks, cudaStream_t s);
 // p4g_sites.cu: the part's site likelihoods from its patterns' lnL, kept as

@@ -569,24 +569,8 @@ k_prune(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks,
 // the program would run (no rescale in between: the values are products of
 // two probabilities, far from FP32's range limits, and a later rescale point
 // scales them by the same exact power of two).
-__device__ __forceinline__ void tipColumn(const PruneJob &J, int leaf, int code, int cat, float *v)
-{
-    const int D = J.dim, NC = J.nCat;
-    if (code < D) {
-        const float *col = J.decks + ((size_t)leaf * NC + cat) * D * D + code * D;
-        for (int i = 0; i < D; i++) v[i] = col[i];
-    } else if (code == D) {
-        for (int i = 0; i < D; i++) v[i] = 1.0f;
-    } else {
-        const float *eq = J.eqTab + (((size_t)leaf * J.nPartial + (code - D - 1)) * NC + cat) * D;
-        for (int i = 0; i < D; i++) v[i] = eq[i];
-    }
-}
-
-// A tip column with the state count known at compile time (float4 reads; the
-// column stays in registers).
 template <int D>
-__device__ __forceinline__ void tipColumnT(const PruneJob &J, int leaf, int code, int cat, float (&v)[D])
+__device__ __forceinline__ void tipColumn(const PruneJob &J, int leaf, int code, int cat, float (&v)[D])
 {
     const int NC = J.nCat;
     if (code < D) {
@@ -627,7 +611,7 @@ constexpr int CHERRY_SLICES = 2, CHERRY_THREADS = 256;
 // staged in shared memory (every thread's rows are the same, so they are read
 // as broadcasts), and the threads take the K x K code pairs.
 template <int D>
-__device__ __forceinline__ void cherryBlockT(const PruneJob &J, int c, int cat, int slice, float *sP)
+__device__ __forceinline__ void cherryBlock(const PruneJob &J, int c, int cat, int slice, float *sP)
 {
     static_assert(D % 4 == 0, "float4 rows");
     const int NC = J.nCat, K = D + 1 + J.nPartial;
@@ -639,8 +623,8 @@ __device__ __forceinline__ void cherryBlockT(const PruneJob &J, int c, int cat, 
     for (int e = slice * CHERRY_THREADS + threadIdx.x; e < K * K; e += CHERRY_SLICES * CHERRY_THREADS) {
         const int ca = e / K, cb = e - ca * K;
         float x[D], y[D];
-        tipColumnT<D>(J, ch.y, ca, cat, x);
-        tipColumnT<D>(J, ch.z, cb, cat, y);
+        tipColumn<D>(J, ch.y, ca, cat, x);
+        tipColumn<D>(J, ch.z, cb, cat, y);
 #pragma unroll
         for (int i = 0; i < D; i++) x[i] = __fmul_rn(x[i], y[i]);
         float4 *out = (float4 *)(J.cherryTab + ((((size_t)c * K + ca) * K + cb) * NC + cat) * D);
@@ -667,29 +651,6 @@ __device__ __forceinline__ void cherryBlockT(const PruneJob &J, int c, int cat, 
     }
 }
 
-// The same for a state count known only at run time.
-__device__ void cherryBlock(const PruneJob &J, int c, int cat, int slice, float *sP)
-{
-    const int D = J.dim, NC = J.nCat, K = D + 1 + J.nPartial;
-    const int4 ch = J.cherries[c];
-    const float *P = J.decks + ((size_t)ch.x * NC + cat) * D * D;
-    for (int k = threadIdx.x; k < D * D; k += blockDim.x) sP[k] = P[k];
-    __syncthreads();
-    for (int e = slice * CHERRY_THREADS + threadIdx.x; e < K * K; e += CHERRY_SLICES * CHERRY_THREADS) {
-        const int ca = e / K, cb = e - ca * K;
-        float x[MAX_DIM], y[MAX_DIM];
-        tipColumn(J, ch.y, ca, cat, x);
-        tipColumn(J, ch.z, cb, cat, y);
-        for (int i = 0; i < D; i++) x[i] = __fmul_rn(x[i], y[i]);
-        float *out = J.cherryTab + ((((size_t)c * K + ca) * K + cb) * NC + cat) * D;
-        for (int s = 0; s < D; s++) {
-            float t = __fmul_rn(sP[s * D], x[0]);
-            for (int j = 1; j < D; j++) t = __fmaf_rn(sP[s * D + j], x[j], t);
-            out[s] = t;
-        }
-    }
-}
-
 // The (job, cherry, category, slice) items of nJobs jobs, spread over the grid:
 // the items are counted in the kernel, CHERRY_THREADS jobs at a time, since a
 // captured launch outlives the topologies it was made for.  (A grid of the
@@ -697,7 +658,7 @@ __device__ void cherryBlock(const PruneJob &J, int c, int cat, int slice, float 
 // 12 parts, most of them without an item: 21 us, this 16.)
 __global__ void __launch_bounds__(CHERRY_THREADS) k_cherry(const PruneJob *__restrict__ jobs, int nJobs)
 {
-    __shared__ __align__(16) float sP[MAX_DIM * MAX_DIM];
+    __shared__ __align__(16) float sP[CHERRY_DIM * CHERRY_DIM];
     __shared__ int sEnd[CHERRY_THREADS], sSum[CHERRY_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31;
     pdlEnter();
@@ -726,8 +687,7 @@ __global__ void __launch_bounds__(CHERRY_THREADS) k_cherry(const PruneJob *__res
             const PruneJob &J = jobs[j0 + k];
             const int at = item - (k ? sEnd[k - 1] : 0);
             const int slice = at % CHERRY_SLICES, u = at / CHERRY_SLICES, c = u / J.nCat, cat = u - c * J.nCat;
-            if (J.dim == 20) cherryBlockT<20>(J, c, cat, slice, sP);
-            else cherryBlock(J, c, cat, slice, sP);
+            cherryBlock<CHERRY_DIM>(J, c, cat, slice, sP);
             __syncthreads();   // sP is free for the next item
         }
         item -= total;
