@@ -155,24 +155,19 @@ enum Op : int { OP_TIPSET = 0, OP_TIPMUL = 1, OP_XFORM = 2, OP_PUSH = 3, OP_MULS
 inline int mkIns(int op, int a, int b) { return op | (a << 4) | (b << 18); }
 
 // Floats of one node's FP32 P decks.  4-state decks hold the categories in
-// pairs (an odd count repeats its last category), 16-byte words of two
-// columns' pairs, [column / 2][pair][row][column % 2][2], the operand order
-// of the paired arithmetic; others are [category][row][column].
-__host__ __device__ constexpr int deckFloats(int dim, int nCat)
-{
-    return dim == 4 ? (nCat + 1) / 2 * 32 : nCat * dim * dim;
-}
+// pairs, 16-byte words of two columns' pairs, [column / 2][pair][row][column % 2][2],
+// the operand order of the paired arithmetic, then an odd count's last category
+// as [row][column]; others are [category][row][column].
+__host__ __device__ constexpr int deckFloats(int dim, int nCat) { return nCat * dim * dim; }
 // Float offset of category cat's (row, column) in a node's 4-state deck.
 __host__ __device__ constexpr int deck4Offset(int nCat, int cat, int row, int col)
 {
-    return (col >> 1) * ((nCat + 1) / 2 * 16) + (cat >> 1) * 16 + row * 4 + (col & 1) * 2 + (cat & 1);
+    return cat < (nCat & ~1) ? (col >> 1) * (nCat / 2 * 16) + (cat >> 1) * 16 + row * 4 + (col & 1) * 2 + (cat & 1)
+                             : nCat / 2 * 32 + row * 4 + col;
 }
 // Floats of one clade-table entry: the categories in pairs too for 4 states,
-// [pair][state][2].
-__host__ __device__ constexpr int entryFloats(int dim, int nCat)
-{
-    return dim == 4 ? (nCat + 1) / 2 * 8 : nCat * dim;
-}
+// [pair][state][2], then an odd count's last, [state].
+__host__ __device__ constexpr int entryFloats(int dim, int nCat) { return nCat * dim; }
 
 // One (tree, part) unit of pruning work, read by every block of that unit.
 struct PruneJob {

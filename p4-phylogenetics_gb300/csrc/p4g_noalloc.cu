@@ -264,12 +264,9 @@ extern "C" int p4g_treeLogLikeNoAlloc(p4g_tree *tt, double *lnL)
         P.isLeaf = (const int *)(g + L.isLeaf);
         P.rates = (double *)(g + L.rates[p]);
         P.eig = (double *)(g + L.eig[p]);
-        // 4-state FP32 decks (categories in pairs) take the FP64 decks' region,
-        // which is large enough for every category count and which nothing
-        // here reads: the array's layout and limit stay what they are
-        P.decks32 = (float *)(g + (dim == 4 ? L.decks64[p] : L.decks32[p]));
+        P.decks32 = (float *)(g + L.decks32[p]);
         P.eqTab = (float *)(g + L.eqTab[p]);
-        P.decks64 = dim == 4 ? nullptr : (double *)(g + L.decks64[p]);
+        P.decks64 = (double *)(g + L.decks64[p]);
         P.partialMask = (const uint32_t *)(g + L.partialMask[p]);
         P.pInvar = mp.pInvar;
         P.relRate = mp.relRate;

@@ -1492,13 +1492,7 @@ __global__ void k_pdeck(const PmatPart *parts, const int *prefix, int nDesc, int
             const float f = __fadd_rn(v.h, v.l);
             const int at = leaf ? j * n + i : i * n + j;   // leaves: column j contiguous
             float *d32 = P.decks32 + (size_t)node * deckFloats(n, P.nCat);
-            if (n == 4) {   // categories in pairs
-                d32 += deck4Offset(P.nCat, cat, at >> 2, at & 3);
-                *d32 = f;
-                if (cat == P.nCat - 1 && (cat & 1) == 0) d32[1] = f;
-            } else {
-                d32[cat * n * n + at] = f;
-            }
+            d32[n == 4 ? deck4Offset(P.nCat, cat, at >> 2, at & 3) : cat * n * n + at] = f;   // categories in pairs
             if (P.decks64)
                 P.decks64[((size_t)node * P.nCat + cat) * n * n + i * n + j] = floatToDouble(v.h) + floatToDouble(v.l);
         }

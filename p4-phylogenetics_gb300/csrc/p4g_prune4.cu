@@ -27,7 +27,11 @@
 //     which its branches and addresses then come from;
 //   - the rescale test's maximum takes three operands an instruction, and the
 //     usual rescale is one product.
-// An odd category count repeats its last category in the pair's upper half.
+// An odd category count's last category is alone: scalar products, its decks and
+// table entries float4 rows behind the pairs'.  (Repeated in a pair's upper half it
+// took two of the FMA pipe's cycles for one value's work and shared memory for
+// two: evaluations of 64 taxa x 115 k patterns x 5 categories 104 us, of 500 taxa
+// x 3 k x 3, whose decks no longer fitted, 490; alone 93 and 186.)
 #include <cuda_runtime.h>
 #include <limits.h>
 #include <algorithm>
@@ -221,15 +225,22 @@ __global__ void __launch_bounds__(TP, MB)
 k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks, int nTiles,
          const int *__restrict__ nTilesDev, int early)
 {
-    constexpr int CPN = (NC + 1) / 2;    // category pairs
+    constexpr int CPN = NC / 2;          // category pairs
+    constexpr bool ODD = NC % 2;         // and a category alone
     static_assert(CPN % G == 0 && (G == 1 || G == 2 || G == 4), "lane groups split the pairs");
-    static_assert(NC % 2 == 0 || G == 1, "an odd category count is not split");
+    static_assert(!ODD || G == 1, "an odd category count is not split");
     constexpr int CPL = CPN / G;         // pairs per lane
     constexpr int NV = CPL * 4;          // pair values per thread and pattern
+    constexpr int CL = 2 * CPL + ODD;    // categories of a lane
     constexpr int TPP = TP / G;
     constexpr int TILE = TPP * PPT;
-    constexpr int DECK = CPN * 32;       // floats of one node's deck
-    constexpr int NQ = NC % 2 ? NC : 2 * CPL;   // 16-byte words of one pattern in a stack slot
+    constexpr int DECK = NC * 16;        // floats of one node's deck: the pairs', then the last category's rows
+    constexpr int ALONE = CPN * 32;      // where those begin
+    constexpr int NQ = CL;               // 16-byte words of one pattern in a stack slot
+    struct Vals {                        // a thread's values of one pattern
+        f2 p[NV ? NV : 1];
+        float s[ODD ? 4 : 1];            // the category alone
+    };
     // the wait on the previous kernel comes before the first read of what it
     // may have written (PDL_EARLY_* bits: what it does not write), so the
     // staging below can run while that kernel drains
@@ -330,13 +341,31 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
         const float *decks = (SDECK ? sDecks : J.decks) + cp0 * 16;
         auto wordOf = [](int i) constexpr -> int { return (i & 1) * (CPN * 64) + (i >> 1) * 64; };
         const uint8_t *myCodes = sCodes + q * PPT;
-        f2 acc[PPT][NV];
+        // the category alone: d = a * v, d = v
+        auto mulAlone = [](float (&d)[ODD ? 4 : 1], const float (&a)[ODD ? 4 : 1], const float4 v) {
+            if constexpr (ODD) {
+                d[0] = __fmul_rn(a[0], v.x);
+                d[1] = __fmul_rn(a[1], v.y);
+                d[2] = __fmul_rn(a[2], v.z);
+                d[3] = __fmul_rn(a[3], v.w);
+            }
+        };
+        auto setAlone = [](float (&d)[ODD ? 4 : 1], const float4 v) {
+            if constexpr (ODD) {
+                d[0] = v.x;
+                d[1] = v.y;
+                d[2] = v.z;
+                d[3] = v.w;
+            }
+        };
+        Vals acc[PPT];
         int E[PPT];
 #pragma unroll
         for (int k = 0; k < PPT; k++) {
             E[k] = 0;
 #pragma unroll
-            for (int i = 0; i < NV; i++) acc[k][i] = pack2(1.f, 1.f);
+            for (int i = 0; i < NV; i++) acc[k].p[i] = pack2(1.f, 1.f);
+            if (ODD) setAlone(acc[k].s, make_float4(1.f, 1.f, 1.f, 1.f));
         }
         auto codesAt = [&](int row) -> int {   // the thread's codes in one row
             if (PPT == 4) return *(const int *)(myCodes + row * TILE);
@@ -348,7 +377,7 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
         // entries before it run.  An entry index at or past the table's end
         // (which a stale or unfilled index row could hold) is not read: entry 0
         // is read instead and oob set.
-        f2 pre[PPT][NV];
+        Vals pre[PPT];
         int preE[PPT];
         int oob = 0;
         auto cladeFetch = [&](int k0) {
@@ -359,13 +388,14 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
                     oob = 1;
                     u = 0;
                 }
-                const float *src = J.cladeTab + ((size_t)u * CPN + cp0) * 8;
+                const float *src = J.cladeTab + (size_t)u * (NC * 4) + cp0 * 8;
 #pragma unroll
                 for (int i = 0; i < NV / 2; i++) {
                     const ulonglong2 w = __ldg((const ulonglong2 *)src + i);
-                    pre[k][2 * i] = w.x;
-                    pre[k][2 * i + 1] = w.y;
+                    pre[k].p[2 * i] = w.x;
+                    pre[k].p[2 * i + 1] = w.y;
                 }
+                if (ODD) setAlone(pre[k].s, __ldg((const float4 *)(src + CPN * 8)));
                 preE[k] = __ldg(J.cladeExp + u);
             }
         };
@@ -378,7 +408,13 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
         auto tipOff = [&](int dk, int c) -> int {
             return c < 4 ? L.offDecks + dk * (DECK * 4) + laneWords + c * 16 : L.offOnes;
         };
-        // The same words for decks read through L1.
+        // the category alone: the row the code selects
+        auto tipAlone = [&](int dk, int c, int off) -> float4 {
+            if (SDECK) return *(const float4 *)(smem + off + ALONE * 4);
+            const float4 v = __ldg((const float4 *)(J.decks + (size_t)dk * DECK + ALONE + (c < 4 ? c : 0) * 4));
+            return c < 4 ? v : make_float4(1.f, 1.f, 1.f, 1.f);
+        };
+        // The pairs' words for decks read through L1.
         auto tipGlobal = [&](int dk, int c, int i) -> ulonglong2 {
             ulonglong2 v = __ldg((const ulonglong2 *)(J.decks + (size_t)dk * DECK + cp0 * 16 + (c < 4 ? c : 0) * 4) + wordOf(i) / 16);
             if (c >= 4) v.x = v.y = pack2(1.f, 1.f);
@@ -386,7 +422,7 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
         };
         auto codeOf = [](int code, int k) -> int { return PPT > 1 ? (code >> (8 * k)) & 0xff : code; };
         // the factor of a partial ambiguity code (sums over its states)
-        auto equate = [&](f2 (&x)[PPT][NV], int dk, int code) {
+        auto equate = [&](Vals (&x)[PPT], int dk, int code) {
             const int node = (SDECK && J.deckMap) ? __ldg(J.deckMap + J.nNodes + dk) : dk;
 #pragma unroll
             for (int k = 0; k < PPT; k++) {
@@ -395,13 +431,15 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
                 const float *eq = J.eqTab + (((size_t)node * J.nPartial + (c - 5)) * NC) * 4;
 #pragma unroll
                 for (int cp = 0; cp < CPL; cp++) {
-                    const int ca = 2 * (cp0 + cp), cb = (NC % 2 && ca == NC - 1) ? ca : ca + 1;
-                    const float4 a = __ldg((const float4 *)eq + ca), b = __ldg((const float4 *)eq + cb);
-                    x[k][4 * cp] = mul2(x[k][4 * cp], pack2(a.x, b.x));
-                    x[k][4 * cp + 1] = mul2(x[k][4 * cp + 1], pack2(a.y, b.y));
-                    x[k][4 * cp + 2] = mul2(x[k][4 * cp + 2], pack2(a.z, b.z));
-                    x[k][4 * cp + 3] = mul2(x[k][4 * cp + 3], pack2(a.w, b.w));
+                    const int ca = 2 * (cp0 + cp);
+                    const float4 a = __ldg((const float4 *)eq + ca), b = __ldg((const float4 *)eq + ca + 1);
+                    f2 *v = x[k].p + 4 * cp;
+                    v[0] = mul2(v[0], pack2(a.x, b.x));
+                    v[1] = mul2(v[1], pack2(a.y, b.y));
+                    v[2] = mul2(v[2], pack2(a.z, b.z));
+                    v[3] = mul2(v[3], pack2(a.w, b.w));
                 }
+                if (ODD) mulAlone(x[k].s, x[k].s, __ldg((const float4 *)eq + NC - 1));
             }
         };
         auto partialCode = [&](int code) -> bool {   // any of the thread's codes a partial ambiguity
@@ -410,12 +448,18 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
             for (int k = 0; k < PPT; k++) any |= codeOf(code, k) > 4;
             return any;
         };
+        auto times = [&](Vals &v, float f) {
+#pragma unroll
+            for (int i = 0; i < NV; i++) v.p[i] = mul2(v.p[i], pack2(f, f));
+            if (ODD) mulAlone(v.s, v.s, make_float4(f, f, f, f));
+        };
         auto rescale = [&]() {
 #pragma unroll
             for (int k = 0; k < PPT; k++) {
                 float mx = 0.f;
 #pragma unroll
-                for (int i = 0; i < NV; i++) mx = max3(mx, lo2(acc[k][i]), hi2(acc[k][i]));
+                for (int i = 0; i < NV; i++) mx = max3(mx, lo2(acc[k].p[i]), hi2(acc[k].p[i]));
+                if constexpr (ODD) mx = max3(max3(mx, acc[k].s[0], acc[k].s[1]), acc[k].s[2], acc[k].s[3]);
 #pragma unroll
                 for (int o = 1; o < G; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
                 if (mx < 0x1p-32f && mx > 0.0f) {
@@ -423,8 +467,7 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
                     if (ex >= 26) {   // one factor 2^k, k = 126 - ex <= 100
                         const float f = __uint_as_float((unsigned)(253 - ex) << 23);
                         E[k] += 126 - ex;
-#pragma unroll
-                        for (int i = 0; i < NV; i++) acc[k][i] = mul2(acc[k][i], pack2(f, f));
+                        times(acc[k], f);
                     } else {
                         int e2;
                         (void)frexp32(mx, &e2);
@@ -432,16 +475,14 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
                         E[k] += x;
                         while (x > 0) {
                             const int step = x > 100 ? 100 : x;
-                            const float f = __uint_as_float((unsigned)(127 + step) << 23);
-#pragma unroll
-                            for (int i = 0; i < NV; i++) acc[k][i] = mul2(acc[k][i], pack2(f, f));
+                            times(acc[k], __uint_as_float((unsigned)(127 + step) << 23));
                             x -= step;
                         }
                     }
                 }
             }
         };
-        auto transform = [&](int deck, f2 (&out)[PPT][NV]) {
+        auto transform = [&](int deck, Vals (&out)[PPT]) {
             const float *P = decks + deck * DECK;
 #pragma unroll
             for (int cp = 0; cp < CPL; cp++)
@@ -451,25 +492,42 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
                                      b = ldPair2<SDECK>(P + wordOf(2 * cp + 1) / 4 + s * 4);
 #pragma unroll
                     for (int k = 0; k < PPT; k++) {
-                        f2 t = mul2(a.x, acc[k][4 * cp]);
-                        t = fma2(a.y, acc[k][4 * cp + 1], t);
-                        t = fma2(b.x, acc[k][4 * cp + 2], t);
-                        out[k][4 * cp + s] = fma2(b.y, acc[k][4 * cp + 3], t);
+                        const f2 *v = acc[k].p + 4 * cp;
+                        f2 t = mul2(a.x, v[0]);
+                        t = fma2(a.y, v[1], t);
+                        t = fma2(b.x, v[2], t);
+                        out[k].p[4 * cp + s] = fma2(b.y, v[3], t);
                     }
                 }
+            if constexpr (ODD) {
+#pragma unroll
+                for (int s = 0; s < 4; s++) {
+                    const float4 *row = (const float4 *)(P + ALONE) + s;
+                    const float4 a = SDECK ? *row : __ldg(row);
+#pragma unroll
+                    for (int k = 0; k < PPT; k++) {
+                        const float *v = acc[k].s;
+                        float t = __fmul_rn(a.x, v[0]);
+                        t = __fmaf_rn(a.y, v[1], t);
+                        t = __fmaf_rn(a.z, v[2], t);
+                        out[k].s[s] = __fmaf_rn(a.w, v[3], t);
+                    }
+                }
+            }
         };
 
         // acc = src * the factor of tip deck dk at the thread's codes
-        auto mulTip = [&](const f2 (&src)[PPT][NV], int dk, int code) {
+        auto mulTip = [&](const Vals (&src)[PPT], int dk, int code) {
 #pragma unroll
             for (int k = 0; k < PPT; k++) {
                 const int c = codeOf(code, k), off = SDECK ? tipOff(dk, c) : 0;
 #pragma unroll
                 for (int i = 0; i < NV / 2; i++) {
                     const ulonglong2 v = SDECK ? *(const ulonglong2 *)(smem + off + wordOf(i)) : tipGlobal(dk, c, i);
-                    acc[k][2 * i] = mul2(src[k][2 * i], v.x);
-                    acc[k][2 * i + 1] = mul2(src[k][2 * i + 1], v.y);
+                    acc[k].p[2 * i] = mul2(src[k].p[2 * i], v.x);
+                    acc[k].p[2 * i + 1] = mul2(src[k].p[2 * i + 1], v.y);
                 }
+                if (ODD) mulAlone(acc[k].s, src[k].s, tipAlone(dk, c, off));
             }
             if (partialCode(code)) equate(acc, dk, code);
         };
@@ -480,45 +538,36 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
 #pragma unroll
                 for (int i = 0; i < NV / 2; i++) {
                     const ulonglong2 v = SDECK ? *(const ulonglong2 *)(smem + off + wordOf(i)) : tipGlobal(dk, c, i);
-                    acc[k][2 * i] = v.x;
-                    acc[k][2 * i + 1] = v.y;
+                    acc[k].p[2 * i] = v.x;
+                    acc[k].p[2 * i + 1] = v.y;
                 }
+                if (ODD) setAlone(acc[k].s, tipAlone(dk, c, off));
             }
             if (partialCode(code)) equate(acc, dk, code);
         };
-        auto mulSlot = [&](const f2 (&src)[PPT][NV], int n) {
+        auto mulSlot = [&](const Vals (&src)[PPT], int n) {
             const float4 *sl = sSlots + n * (NC * TILE) + tid;
 #pragma unroll
-            for (int k = 0; k < PPT; k++)
+            for (int k = 0; k < PPT; k++) {
 #pragma unroll
-                for (int i = 0; i < NQ; i++) {
-                    const int w = k * NQ + i;
-                    if (NC % 2 && i == NQ - 1) {   // the odd category alone
-                        const float4 v = sl[w * TP];
-                        acc[k][NV - 4] = mul2(src[k][NV - 4], pack2(v.x, v.x));
-                        acc[k][NV - 3] = mul2(src[k][NV - 3], pack2(v.y, v.y));
-                        acc[k][NV - 2] = mul2(src[k][NV - 2], pack2(v.z, v.z));
-                        acc[k][NV - 1] = mul2(src[k][NV - 1], pack2(v.w, v.w));
-                    } else {
-                        const ulonglong2 v = *(const ulonglong2 *)(sl + w * TP);
-                        acc[k][2 * i] = mul2(src[k][2 * i], v.x);
-                        acc[k][2 * i + 1] = mul2(src[k][2 * i + 1], v.y);
-                    }
+                for (int i = 0; i < NV / 2; i++) {
+                    const ulonglong2 v = *(const ulonglong2 *)(sl + (k * NQ + i) * TP);
+                    acc[k].p[2 * i] = mul2(src[k].p[2 * i], v.x);
+                    acc[k].p[2 * i + 1] = mul2(src[k].p[2 * i + 1], v.y);
                 }
+                if (ODD) mulAlone(acc[k].s, src[k].s, sl[(k * NQ + NQ - 1) * TP]);
+            }
         };
-        auto pushSlot = [&](const f2 (&src)[PPT][NV], int n) {
+        auto pushSlot = [&](const Vals (&src)[PPT], int n) {
             float4 *sl = sSlots + n * (NC * TILE) + tid;
 #pragma unroll
-            for (int k = 0; k < PPT; k++)
+            for (int k = 0; k < PPT; k++) {
 #pragma unroll
-                for (int i = 0; i < NQ; i++) {
-                    const int w = k * NQ + i;
-                    if (NC % 2 && i == NQ - 1)
-                        sl[w * TP] = make_float4(lo2(src[k][NV - 4]), lo2(src[k][NV - 3]), lo2(src[k][NV - 2]),
-                                                 lo2(src[k][NV - 1]));
-                    else
-                        *(ulonglong2 *)(sl + w * TP) = make_ulonglong2(src[k][2 * i], src[k][2 * i + 1]);
-                }
+                for (int i = 0; i < NV / 2; i++)
+                    *(ulonglong2 *)(sl + (k * NQ + i) * TP) = make_ulonglong2(src[k].p[2 * i], src[k].p[2 * i + 1]);
+                if constexpr (ODD)
+                    sl[(k * NQ + NQ - 1) * TP] = make_float4(src[k].s[0], src[k].s[1], src[k].s[2], src[k].s[3]);
+            }
         };
 
         const int nEntries = sCount;
@@ -537,7 +586,7 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
             const int3 In = entryAt(ip + 1);
             const int what = I.x & 63, dk = I.y & 0xffff;
             if (what & F4_MAIN) {   // the entries of a binary tree
-                f2 x[PPT][NV];
+                Vals x[PPT];
                 rescale();
                 transform((unsigned)I.x >> DECK4_SHIFT, x);
                 if (what & F4_TIP) {
@@ -553,21 +602,18 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
                 }
             } else {
                 if (what & F4_XFORM) {
-                    f2 x[PPT][NV];
+                    Vals x[PPT];
                     rescale();
                     transform((unsigned)I.x >> DECK4_SHIFT, x);
 #pragma unroll
-                    for (int k = 0; k < PPT; k++)
-#pragma unroll
-                        for (int i = 0; i < NV; i++) acc[k][i] = x[k][i];
+                    for (int k = 0; k < PPT; k++) acc[k] = x[k];
                 }
                 if (I.x & F4_PUSH) pushSlot(acc, (I.x >> SLOT4_SHIFT) & 0x1ff);
                 if (what & F4_START) setTip((unsigned)I.y >> 16, codeS);
                 if (what & F4_CLADE) {
 #pragma unroll
                     for (int k = 0; k < PPT; k++) {
-#pragma unroll
-                        for (int i = 0; i < NV; i++) acc[k][i] = pre[k][i];
+                        acc[k] = pre[k];
                         E[k] += preE[k];
                     }
                     if (++nextClade < J.nClade) cladeFetch(nextClade);
@@ -581,22 +627,22 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
         }
         rescale();   // the last node's; a clade's values go through its edge's transform
         if (J.cladeOut) {
-            f2 out[PPT][NV];
+            Vals out[PPT];
             transform((__ldg(J.prog + J.nProg - 1) >> 4) & 0x3fff, out);
 #pragma unroll
-            for (int k = 0; k < PPT; k++)
-#pragma unroll
-                for (int i = 0; i < NV; i++) acc[k][i] = out[k][i];
+            for (int k = 0; k < PPT; k++) acc[k] = out[k];
         }
 
         if (J.cladeOut) {   // clade-table job: the transformed product and its exponent
 #pragma unroll
             for (int k = 0; k < PPT; k++) {
                 if (!valid[k]) continue;
-                float *o = J.cladeOut + ((size_t)pp[k] * CPN + cp0) * 8;
+                float *o = J.cladeOut + (size_t)pp[k] * (NC * 4) + cp0 * 8;
 #pragma unroll
                 for (int i = 0; i < NV / 2; i++)
-                    *((ulonglong2 *)o + i) = make_ulonglong2(acc[k][2 * i], acc[k][2 * i + 1]);
+                    *((ulonglong2 *)o + i) = make_ulonglong2(acc[k].p[2 * i], acc[k].p[2 * i + 1]);
+                if constexpr (ODD)
+                    *(float4 *)(o + CPN * 8) = make_float4(acc[k].s[0], acc[k].s[1], acc[k].s[2], acc[k].s[3]);
                 if (g == 0) J.cladeOutExp[pp[k]] = E[k];
             }
             continue;
@@ -609,12 +655,12 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
         const int lane = tid & 31;
         const int base = lane & ~(G - 1);
         const int rootRow = (J.rootLeafRow >= 0 && J.rowMap) ? J.rowMap[J.rootLeafRow] : J.rootLeafRow;
-        // category c of this lane (c = 0 .. 2 CPL - 1; an odd count's last pair holds one)
+        // category c of this lane
         auto val = [&](int k, int c, int s) -> float {
-            const f2 w = acc[k][4 * (c >> 1) + s];
+            if (ODD && c == CL - 1) return acc[k].s[ODD ? s : 0];
+            const f2 w = acc[k].p[4 * (c >> 1) + s];
             return (c & 1) ? hi2(w) : lo2(w);
         };
-        constexpr int CL = NC % 2 ? NC : 2 * CPL;   // categories of this lane
 #pragma unroll
         for (int k = 0; k < PPT; k++) {
             uint32_t rmask = 15u;
@@ -739,9 +785,9 @@ constexpr int kSmallOdd4 = 13, kSmallEven4 = 8;
 
 // Where a caller may ask for a shape: (threads, tile, decks staged) as the
 // numbers were first given out, 16 floats a deck and category.  The forms above
-// hold more for some of them (decks in category pairs, decks staged where they
-// were not, larger tiles); a tree that the first form fits and today's does not
-// runs the smallest shape.  (Refused instead, shapes 6 and 10 were lost from 500
+// hold more for some of them (a row of ones, decks staged where they were not); a
+// tree that the first form fits and today's does not runs the smallest shape.
+// (Refused instead, shapes 6 and 10 were lost from 500
 // taxa on and a tree of 800 taxa and one category could not be evaluated.)
 struct First4 {
     int tp, tile;

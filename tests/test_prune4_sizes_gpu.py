@@ -71,6 +71,26 @@ def test_shapes_can_be_pinned_where_they_could(nCat, kind, n, lib):
     e.free()
 
 
+@pytest.mark.parametrize("nCat,n", [(1, 600), (3, 320), (5, 210)])
+def test_odd_counts_take_no_more_than_their_categories(nCat, n, lib):
+    """A staged shape that fits with 16 floats a category (and a row of ones) runs
+    itself, not a smaller one in its place."""
+    e = _engine("yule", n, nCat)
+    pf.setCladeSize(e.cTree, 0)
+    lnl = e.calcLogLike()
+    info = pf.treeInfo(e.cTree)
+    for shape in (0, 1, 2):
+        threads, tile, _, _ = FIRST[shape]
+        need = info["nProg"] * 16 + (e.problem.tree.nNodes + 1) * nCat * 64 + (n * tile + 15) // 16 * 16 + 16 \
+            + info["nSlots"] * nCat * 16 * tile + threads // 32 * 8 + 16
+        assert shape != 0 or need <= 227 * 1024
+        if need <= 227 * 1024:
+            pf.setPruneShape(e.cTree, 0, shape)
+            assert pf.getPruneShape(e.cTree, 0) == (shape, tile)
+            assert abs(e.calcLogLike() - lnl) <= 1e-12 * abs(lnl), shape
+    e.free()
+
+
 @pytest.mark.parametrize("nCat", [1, 3, 5])
 def test_the_smallest_shape_of_odd_counts(nCat, lib):
     e = _engine("yule", 60, nCat)
