@@ -12,6 +12,7 @@
 // Every iteration is capped; a non-converging input returns an error.
 #pragma once
 #include <math.h>
+#include <string.h>
 
 #ifdef __CUDACC__
 #define P4G_HD __host__ __device__
@@ -237,28 +238,33 @@ P4G_HD inline double gm_chi2Quantile(double prob, double v)
     return -1.0;
 }
 
-#ifdef __CUDACC__
 // e^x in FP64 with a short dependence chain (this GPU's FP64 latency, not its
 // rate, is what a few exponentials cost: a Newton step's 5.4 k clocks with
-// exp(), 3.2 k with this): x = k ln2 + r with ln2 in two parts, e^r by its
-// Taylor series to r^13 / 13! (|r| <= ln2 / 2: the rest is below 4e-18) in Estrin's order, scaled
-// by 2^k.  Within 2 ulp of exp(); results below the normal range are 0.
-__device__ __forceinline__ double expShort(double x)
+// exp(), 3.2 k with this).  x = k ln2 + r with ln2 in two parts, the first of 41
+// bits, so that its product with k and the difference are exact; e^r - 1 by its
+// Taylor series to r^13 / 13! (|r| <= ln2 / 2: the rest is below 5e-18) in
+// Estrin's order; the 1 and the 2^k in the last FMA.  Three roundings of up to
+// 2^-55 and smaller ones before the last: within 1.5 ulp of e^x for -708 <= x < 700 (with
+// 1 + r formed first, as in a plain Estrin sum, it was 2.004).  Below, where e^x is
+// under 3.4e-308, 0.
+P4G_HD inline double expShort(double x)
 {
     if (!(x < 700.0)) return exp(x);
     if (x < -708.0) return 0.0;
     const double k = rint(x * 1.4426950408889634074);
-    double r = fma(-k, 0.69314718055994530942, x);
-    r = fma(-k, 2.3190468138462995584e-17, r);
-    const double r2 = r * r, r4 = r2 * r2, r8 = r4 * r4;
-    const double a0 = 1.0 + r, a1 = fma(1.0 / 6.0, r, 0.5), a2 = fma(1.0 / 120.0, r, 1.0 / 24.0),
+    double r = fma(-k, 0.69314718055966295651160180568695068359375, x);
+    r = fma(-k, 2.82352905630315771225884481750134360e-13, r);
+    const double r2 = r * r, r4 = r2 * r2, r6 = r4 * r2;
+    const double a1 = fma(1.0 / 6.0, r, 0.5), a2 = fma(1.0 / 120.0, r, 1.0 / 24.0),
                  a3 = fma(1.0 / 5040.0, r, 1.0 / 720.0), a4 = fma(1.0 / 362880.0, r, 1.0 / 40320.0),
                  a5 = fma(1.0 / 39916800.0, r, 1.0 / 3628800.0), a6 = fma(1.0 / 6227020800.0, r, 1.0 / 479001600.0);
-    const double b0 = fma(a1, r2, a0), b1 = fma(a3, r2, a2), b2 = fma(a5, r2, a4);
-    const double c0 = fma(b1, r4, b0), c1 = fma(a6, r4, b2);
-    return fma(c1, r8, c0) * __longlong_as_double((long long)((int)k + 1023) << 52);
+    const double b1 = fma(a2, r2, a1), b2 = fma(a4, r2, a3), b3 = fma(a6, r2, a5);
+    const double s = fma(fma(b3, r4, b2), r6, fma(b1, r2, r));
+    const long long bits = ((long long)(int)k + 1023) << 52;
+    double scale;
+    memcpy(&scale, &bits, sizeof(scale));
+    return fma(s, scale, scale);
 }
-#endif
 
 // K equal-probability categories of Gamma(alpha, alpha), rate = bin mean.
 // cut[] is caller scratch of K entries.  Returns 0 or -1.
