@@ -774,7 +774,7 @@ def main():
     nClades = pf.treeInfo(eng.cTree).get("nClade", 0)   # before the batch below (batches use none)
     cl = 1 if nClades else 0
 
-    # ---- the plain FP64 GPU path (per-node launches), same steps, L2 flushed
+    # ---- the plain FP64 GPU path (one launch a part), same steps, L2 flushed
     pf.setPrecision(eng.cTree, 1)
     for _ in range(3):
         pf.treeLogLikeAsync(eng.cTree, 1)
@@ -852,16 +852,16 @@ def main():
     fbytes = fused_bytes(problem)
     traffic = read_traffic(args.config)
     tflops = flops / (prune_ms * 1e-3) / 1e12
-    kname = ("k_prune_tc" if (sp0.dim == 20 and shape == 3) else "k_prune")
-    if kname == "k_prune":
+    kname = "k_prune_tc" if (sp0.dim == 20 and shape == 3) else "k_prune4" if sp0.dim == 4 else "k_prune"
+    if kname != "k_prune_tc":
         roof = {"bound": "fp32", "achieved": tflops,
                 "peak": fp32_peak["tflops"], "unit": "TFLOP/s", "frac": tflops / fp32_peak["tflops"],
                 "traffic": traffic,
                 "peak_source": "measured FP32 FMA throughput on this GPU (p4g_fp32FmaPeak, CUDA events, SM clock "
                                "%s MHz sampled during the probe), frac of measured" % fp32_peak["sm_mhz"],
-                "binding_resource": "FP32 issue and latency on the CUDA cores (ncu: issue active < 45 %, long-"
-                                    "scoreboard stalls on the clade-table gathers, 14-15 warps per SM for one "
-                                    "tree); the kernel keeps every conditional likelihood on chip, so HBM does "
+                "binding_resource": "FP32 issue and latency on the CUDA cores (ncu: issue active < 45 %, "
+                                    "stalls on the shared-memory decks and the clade-table gathers, 14-15 warps "
+                                    "per SM for one tree); the kernel keeps every conditional likelihood on chip, so HBM does "
                                     "not bind it"}
     else:   # split-TF32 tensor-core kernel: TF32 dense runs at half the measured bf16 rate
         tf32 = measured_peak("bf16_tflops", 1900.0) / 2.0
@@ -873,7 +873,7 @@ def main():
                 "fp32_equivalent": {"peak": fp32_peak["tflops"], "frac": tflops / fp32_peak["tflops"],
                                     "note": "the same flops against the measured FP32 FMA throughput"},
                 "binding_resource": "latency between the four warpgroups' MMA issue, commit wait and TMEM read-"
-                                    "back (ncu: tensor pipe active ~3 %, issue active ~31 %, long-scoreboard and "
+                                    "back (ncu: tensor pipe active ~10 %, issue active ~31 %, long-scoreboard and "
                                     "barrier stalls); the leaf gathers and products run on the CUDA cores"}
     roof.update({
             "kernel": "%s<D=%d,nCat=%d> fused pruning + root log-sum (tile shape %d: %d patterns "
@@ -907,11 +907,11 @@ def main():
                             "parameter image is copied only when other values change)"},
             "gpu_launches": args.steps * (2 + 1 + 2 + 3 * cl) + nfull * (3 + cl)
             + n64 * (1 + len(problem.parts)) + nbSteps * 3,
-            "gpu_launches_note": "value step: k_pdeck + k_prune (+ the clade-table k_prune when clade tables "
-                                 "are on); prune-only: k_prune (+ clade tables); e2e: k_pdeck + k_prune "
+            "gpu_launches_note": "value step: k_pdeck + k_prune4 (+ the clade-table k_prune4 when clade tables "
+                                 "are on); prune-only: k_prune4 (+ clade tables); e2e: k_pdeck + k_prune4 "
                                  "(+ clade tables); full step adds k_gammaEig; FP64 step: k_pdeck + one "
                                  "k_prune64 per part; batched step (graph): k_gammaEig + "
-                                 "k_pdeck + k_prune",
+                                 "k_pdeck + k_prune4",
             "full_setprams": {"value": 1e3 / full_ms, "unit": "evals/s", "ms_per_step": full_ms,
                               "note": "comps, R, gamma shape and branch lengths all change every step: every "
                                       "eigensystem and gamma rate set is recomputed"},

@@ -264,10 +264,10 @@ struct TreeDev {
     bool rootCLOn = false, jobsRootCL = false;   // root partials wanted / in the jobs
     // nParts lnLs, then the status int: the kernels write them here (hOutDev),
     // in host memory, so an evaluation ends with its last kernel.  A copy
-    // from device memory behind it cost up to 12 us more: the copy engine
-    // starts on a period of about 12 us after a kernel (measured: kernel +
-    // copy + synchronise 23, 35, 47, 59 us for kernels of 5 to 45 us; with the
-    // kernel's own store 13 us + the kernel).
+    // from device memory behind it cost up to 9 us more: the copy engine
+    // starts on a period of about 12 us after a kernel (launch to synchronised,
+    // kernels of 4, 8, 12, 21, 31, 45 us: 13, 22, 22, 35, 47, 59 us with a copy, 10,
+    // 14, 18, 27, 37, 50 with the kernel's own store).
     PinnedBuf hOut;
     void *hOutDev = nullptr;
     cudaEvent_t imgFree = nullptr;   // last H2D of the image done

@@ -300,7 +300,8 @@ __device__ void stepChunk(const NewtPart &A, const double *sE, double (*sLike)[k
     }
 }
 
-// BIG: parts of 20 states among them (their code alone takes 254 registers).
+// BIG: parts of 20 states among them (with their code the kernel takes 168
+// registers and spills 53 words, without it 96 and 37).
 template <bool BIG>
 __global__ void __launch_bounds__(kBlock) k_newtRound(NewtRound G)
 {
