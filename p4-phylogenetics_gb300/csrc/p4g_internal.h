@@ -5,6 +5,7 @@
 #include <stdint.h>
 #include <functional>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 #include "p4gpu.h"
@@ -82,10 +83,12 @@ struct Part {
     int upload(cudaStream_t s);
     DevBuf dSeqPos;               // seqPosIdx [nChar], of the data uploaded as generation sitesGen
     unsigned long long sitesGen = 0;
+    std::mutex sitesLock;         // dSeqPos and hSiteLikes, while they are made
     int uploadSites(cudaStream_t s);
     // ancestral-state draws (p4g_sim.cu): the caller's uniforms and the draws,
     // in use during a call alone, so that the data and not each of their
-    // trees hold the 24 bytes a site
+    // trees hold the 24 bytes a site; drawLock: one call at a time
+    std::mutex drawLock;
     DevBuf dUniforms;
     PinnedBuf hDraws;
 };

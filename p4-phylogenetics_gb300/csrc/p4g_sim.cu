@@ -252,7 +252,9 @@ extern "C" int p4g_drawAncStates(p4g_tree *tt, int pNum, const double *uniforms,
     const ModelPart &mp = t->model->parts[pNum];
     Part *dp = t->data->parts[pNum];
     const int nChar = dp->nChar;
-    // the draws land in a host buffer the data keep, the failure flag behind them
+    // the draws land in a host buffer the data keep, the failure flag behind them;
+    // threads that draw on trees of the same data take turns with it
+    std::lock_guard<std::mutex> hold(dp->drawLock);
     const size_t drawBytes = sizeof(int) * 4 * (size_t)nChar;
     RET(dp->hDraws.ensure(drawBytes + 16));
     void *hDev = nullptr;

@@ -50,6 +50,7 @@ __global__ void __launch_bounds__(1024) k_siteLikes(const double *__restrict__ l
 
 int Part::uploadSites(cudaStream_t s)
 {
+    std::lock_guard<std::mutex> hold(sitesLock);
     if (sitesGen == gen && dSeqPos.ptr) return P4G_OK;
     RET(dSeqPos.ensure(sizeof(int) * std::max(nChar, 1)));
     P4G_CUDA(cudaMemcpyAsync(dSeqPos.ptr, seqPosIdx.data(), sizeof(int) * nChar, cudaMemcpyHostToDevice, s));
@@ -60,9 +61,12 @@ int Part::uploadSites(cudaStream_t s)
 int launchSiteLikes(Part *p, const double *dLnl, const double *partLnl, int nParts, const int *status, cudaStream_t s)
 {
     RET(p->uploadSites(s));
-    RET(p->hSiteLikes.ensure(sizeof(double) * std::max(p->nChar, 1)));
     void *out = nullptr;
-    RET(p->hSiteLikes.device(&out));
+    {
+        std::lock_guard<std::mutex> hold(p->sitesLock);
+        RET(p->hSiteLikes.ensure(sizeof(double) * std::max(p->nChar, 1)));
+        RET(p->hSiteLikes.device(&out));
+    }
     if (p->nChar <= 0) return P4G_OK;
     // a block per SM with an even share of the sites, since every block loads
     // the words in host memory: 400,000 sites took 433 us an evaluation with eight
