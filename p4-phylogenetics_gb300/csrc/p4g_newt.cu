@@ -28,7 +28,7 @@
 // What bounds it: the chain of Newton steps (exponentials, FP64 sums, a grid
 // barrier of about 1.5 us each).  With a host round trip per step (two
 // launches, a copy, a synchronisation) a whole optimisation of 32 taxa x 10,000
-// sites took 99 ms; with the schedule on the device 23 ms.
+// sites took 101 ms; with the schedule on the device 24 ms.
 //
 // cl2 is stored for every node as [nNodes][nCat][dim][nPatPad] FP64 beside
 // the FP64 path's cl of the internal nodes.
