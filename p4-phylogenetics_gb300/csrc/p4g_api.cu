@@ -1327,6 +1327,7 @@ static int refreshProgram(Tree *t)
         if (jobs[p].cherryTab)
             dv.cherryWork = std::max(dv.cherryWork, (long long)dv.cherryList.size() * jobs[p].nCat);
     }
+    bool retiled = false;
     for (auto &g : dv.groups) {
         g.smem = pruneSmemBytes(g.dim, g.nCat, dv.nProg, t->nNodes, t->data->nTax, dv.nSlots, g.shape,
                                 dv.nClade, dv.nDeck, dv.nRow);
@@ -1339,8 +1340,10 @@ static int refreshProgram(Tree *t)
                                 "tree too large for the fused kernel's shared memory (%d bytes)", g.smem);
             g.shape = best;
             g.smem = bestSmem;
+            retiled = true;
         }
     }
+    if (retiled) RET(layoutBlocks(t));   // the tiles of the shape that now runs
     dv.progDirty = false;
     return P4G_OK;
 }
