@@ -2316,7 +2316,11 @@ extern "C" int p4g_treeInfo(p4g_tree *tt, long long *info)
     if (!t || !info) return setError(P4G_EINVAL, "treeInfo: null argument");
     RET(validateModel(t, -1));
     RET(allocTreeDev(t));
-    RET(refreshProgram(t));
+    if (t->dev.progDirty) {   // on the device too: an evaluation without setPrams may follow
+        RET(waitImage(t));
+        RET(refreshProgram(t));
+        if (t->dev.haveParams) RET(uploadImage(t));
+    }
     int launches = (int)t->dev.groups.size();
     int nG = 0, nE = 0, nD = 0;
     long long nPat = 0;
