@@ -1675,7 +1675,7 @@ static int autotune(Tree *t, bool fresh = false)
         std::vector<float> shapeMs(nShapes, 1e30f);
         for (int round = 0; round < 2; round++)
             for (int sh = 0; sh < nShapes; sh++) {
-                if (!pruneShapeValid(gr.dim, gr.nCat, sh)) continue;
+                if (!pruneShapeTimed(gr.dim, gr.nCat, sh, t->nNodes)) continue;
                 gr.shape = sh;
                 gr.smem = pruneSmemBytes(gr.dim, gr.nCat, dv.nProg, t->nNodes, t->data->nTax, dv.nSlots, sh,
                                          dv.nClade, dv.nDeck, dv.nRow);
@@ -1795,7 +1795,7 @@ static int tuneCladeShapes(Tree *t)
         const int key = k.first * 64 + k.second;
         std::vector<int> cand;
         for (int sh = 0; sh < pruneNumShapes(k.first); sh++)
-            if (pruneShapeValid(k.first, k.second, sh)) cand.push_back(sh);
+            if (pruneShapeTimed(k.first, k.second, sh, t->nNodes)) cand.push_back(sh);
         std::vector<float> best(cand.size(), 1e30f);
         for (int round = 0; round < 2; round++)
             for (size_t c = 0; c < cand.size(); c++) {
@@ -3075,7 +3075,7 @@ static int batchTune(Batch *b)
         int best = keep;
         float bestMs = 1e30f;
         for (int sh = 0; sh < pruneNumShapes(dim); sh++) {
-            if (!pruneShapeValid(dim, nCat, sh)) continue;
+            if (!pruneShapeTimed(dim, nCat, sh, b->trees[0]->nNodes)) continue;
             bool fits = true;
             for (Tree *t : b->trees) {
                 TreeDev &dv = t->dev;

@@ -253,11 +253,7 @@ int cladeBuild(Tree *t, const std::vector<int> &need, const std::vector<int> &cl
     }
     std::vector<int> shapeOfGroup(keys.size()), tileOfGroup(keys.size());
     for (size_t gi = 0; gi < keys.size(); gi++) {
-        // the combination counts are small: lane groups of 2 split the
-        // categories so that the tables spread over more blocks; P decks are
-        // read through L1 (a clade touches few of them)
-        int shape = defaultShape(keys[gi].first);
-        if (keys[gi].first == 4) shape = keys[gi].second % 2 == 0 ? 8 : 3;
+        int shape = keys[gi].first == 4 ? prune4CladeShape(keys[gi].second, nn) : defaultShape(keys[gi].first);
         auto it = dv.cladeShape.find(keys[gi].first * 64 + keys[gi].second);   // chosen by the timing
         if (it != dv.cladeShape.end()) {
             int bytes = 0;

@@ -408,6 +408,7 @@ int launchPrune(const PruneJob *dJobs, const BlockDesc *dBlocks, int nTiles, int
 int pruneNumShapes(int dim);
 int pruneTile(int dim, int nCat, int shape);
 int pruneShapeValid(int dim, int nCat, int shape);
+int pruneShapeTimed(int dim, int nCat, int shape, int nNodes);   // a choice of the autotuner's
 int pruneKernelExists(int dim, int nCat, int shape);
 constexpr int CHERRY_DIM = 20;   // states of the parts that have cherry tables
 // cherryBlocks: cherry-list length (or capacity) x the largest nCat of the parts with tables
@@ -420,7 +421,9 @@ int prune4NumShapes();
 int prune4ShapeValid(int nCat, int shape);
 int prune4KernelExists(int nCat, int shape);
 int prune4Tile(int nCat, int shape);
-int prune4Smallest(int nCat);
+int prune4ShapeTimed(int nCat, int shape, int nNodes);
+int prune4Smallest(int nCat, int nNodes);
+int prune4CladeShape(int nCat, int nNodes);
 int prune4SmemBytes(int nCat, int nProg, int nDecks, int nRows, int nSlots, int shape, int nClade);
 int prune4FirstBytes(int nCat, int nProg, int nDecks, int nRows, int nSlots, int shape, int nClade);
 int launchPrune4(const PruneJob *dJobs, const BlockDesc *dBlocks, int nTiles, int nCat, int smemBytes, int shape,

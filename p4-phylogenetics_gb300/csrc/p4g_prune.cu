@@ -742,6 +742,11 @@ int pruneShapeValid(int dim, int nCat, int shape)
     return nCat % shapeOf(dim, shape).g == 0;
 }
 
+int pruneShapeTimed(int dim, int nCat, int shape, int nNodes)
+{
+    return dim == 4 ? prune4ShapeTimed(nCat, shape, nNodes) : pruneShapeValid(dim, nCat, shape);
+}
+
 int pruneTile(int dim, int nCat, int shape)
 {
     if (dim == 4) return prune4Tile(nCat, shape);
@@ -765,7 +770,7 @@ int pruneSmemBytes(int dim, int nCat, int nProg, int nNodes, int nTax, int nSlot
 int pruneShapeSmallest(int dim, int nCat, int nProg, int nNodes, int nTax, int nSlots, int nClade, int nDeck, int nRow,
                        int *bytes)
 {
-    int best = dim == 4 ? prune4Smallest(nCat) : 0;
+    int best = dim == 4 ? prune4Smallest(nCat, nNodes) : 0;
     *bytes = pruneSmemBytes(dim, nCat, nProg, nNodes, nTax, nSlots, best, nClade, nDeck, nRow);
     for (int sh = 0; sh < pruneNumShapes(dim); sh++) {
         if (!pruneShapeValid(dim, nCat, sh)) continue;

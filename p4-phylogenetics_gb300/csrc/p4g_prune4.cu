@@ -217,8 +217,9 @@ __device__ void decodeProgram4(const PruneJob &J, int4 *out, int *count, const i
 // One block walks tiles blockIdx.x, +gridDim.x, ...; the job's program and
 // P decks are staged once per job change, the tip codes once per tile.
 // A pattern is handled by G adjacent lanes, lane g holding the category pairs
-// [g * CPL, (g + 1) * CPL); a thread works on PPT adjacent patterns, whose
-// transforms share every P load.
+// [g * CPL, (g + 1) * CPL), or where G does not divide them (shapes 14 and 15) the
+// last CPL, a pair then being formed by two lanes; a thread works on PPT adjacent
+// patterns, whose transforms share every P load.
 // MB: resident blocks per SM the registers are held to (0: free).
 template <int NC, int TP, int PPT, bool SDECK, int G, int MB>
 __global__ void __launch_bounds__(TP, MB)
@@ -227,16 +228,17 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
 {
     constexpr int CPN = NC / 2;          // category pairs
     constexpr bool ODD = NC % 2;         // and a category alone
-    static_assert(CPN % G == 0 && (G == 1 || G == 2 || G == 4), "lane groups split the pairs");
+    static_assert(CPN >= G || G == 1, "every lane has a pair of its own");
     static_assert(!ODD || G == 1, "an odd category count is not split");
-    constexpr int CPL = CPN / G;         // pairs per lane
+    constexpr int CPL = (CPN + G - 1) / G;   // pairs per lane
+    constexpr bool SHARED_PAIR = CPL * G != CPN;
     constexpr int NV = CPL * 4;          // pair values per thread and pattern
     constexpr int CL = 2 * CPL + ODD;    // categories of a lane
     constexpr int TPP = TP / G;
     constexpr int TILE = TPP * PPT;
     constexpr int DECK = NC * 16;        // floats of one node's deck: the pairs', then the last category's rows
     constexpr int ALONE = CPN * 32;      // where those begin
-    constexpr int NQ = CL;               // 16-byte words of one pattern in a stack slot
+    constexpr int NQ = CL;               // a lane's 16-byte words of one pattern in a stack slot
     struct Vals {                        // a thread's values of one pattern
         f2 p[NV ? NV : 1];
         float s[ODD ? 4 : 1];            // the category alone
@@ -257,7 +259,12 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
     asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));   // read once
     const int q = tid / G;               // thread's pattern group in the tile
     const int g = tid % G;               // lane in the group
-    const int cp0 = g * CPL;             // first category pair of this lane
+    const int cp0 = SHARED_PAIR ? min(g * CPL, CPN - CPL) : g * CPL;   // first category pair of this lane
+    // the lane's word i of its k-th pattern in a stack slot; lanes that form the same
+    // pair store the same words and read only what they stored
+    auto slotWord = [&](int k, int i) -> int {
+        return SHARED_PAIR ? (k * NC + 2 * cp0 + i) * TPP + q : (k * NQ + i) * TP + tid;
+    };
     __shared__ int sLast, sCount;
     int curJob = -1;
     Layout4 L;
@@ -546,27 +553,27 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
             if (partialCode(code)) equate(acc, dk, code);
         };
         auto mulSlot = [&](const Vals (&src)[PPT], int n) {
-            const float4 *sl = sSlots + n * (NC * TILE) + tid;
+            const float4 *sl = sSlots + n * (NC * TILE);
 #pragma unroll
             for (int k = 0; k < PPT; k++) {
 #pragma unroll
                 for (int i = 0; i < NV / 2; i++) {
-                    const ulonglong2 v = *(const ulonglong2 *)(sl + (k * NQ + i) * TP);
+                    const ulonglong2 v = *(const ulonglong2 *)(sl + slotWord(k, i));
                     acc[k].p[2 * i] = mul2(src[k].p[2 * i], v.x);
                     acc[k].p[2 * i + 1] = mul2(src[k].p[2 * i + 1], v.y);
                 }
-                if (ODD) mulAlone(acc[k].s, src[k].s, sl[(k * NQ + NQ - 1) * TP]);
+                if (ODD) mulAlone(acc[k].s, src[k].s, sl[slotWord(k, NQ - 1)]);
             }
         };
         auto pushSlot = [&](const Vals (&src)[PPT], int n) {
-            float4 *sl = sSlots + n * (NC * TILE) + tid;
+            float4 *sl = sSlots + n * (NC * TILE);
 #pragma unroll
             for (int k = 0; k < PPT; k++) {
 #pragma unroll
                 for (int i = 0; i < NV / 2; i++)
-                    *(ulonglong2 *)(sl + (k * NQ + i) * TP) = make_ulonglong2(src[k].p[2 * i], src[k].p[2 * i + 1]);
+                    *(ulonglong2 *)(sl + slotWord(k, i)) = make_ulonglong2(src[k].p[2 * i], src[k].p[2 * i + 1]);
                 if constexpr (ODD)
-                    sl[(k * NQ + NQ - 1) * TP] = make_float4(src[k].s[0], src[k].s[1], src[k].s[2], src[k].s[3]);
+                    sl[slotWord(k, NQ - 1)] = make_float4(src[k].s[0], src[k].s[1], src[k].s[2], src[k].s[3]);
             }
         };
 
@@ -674,10 +681,12 @@ k_prune4(const PruneJob *__restrict__ jobs, const BlockDesc *__restrict__ blocks
             for (int j = 0; j < G; j++) {
                 if (g == j) {
 #pragma unroll
-                    for (int c = 0; c < CL; c++)
+                    for (int c = 0; c < CL; c++) {
+                        if (SHARED_PAIR && 2 * cp0 + c < 2 * CPL * j) continue;   // the lane before has it
 #pragma unroll
                         for (int s = 0; s < 4; s++)
                             if ((rmask >> s) & 1u) like32 = __fmaf_rn(sPi[s], val(k, c, s), like32);
+                    }
                 }
                 if (G > 1 && j < G - 1) {
                     const float nxt = __shfl_sync(0xffffffffu, like32, base + j);
@@ -770,8 +779,8 @@ struct Shape4 {
     int g, mb, div;
     bool only34;
 };
-// every tile holds 64 to 512 patterns; the last shape, for odd counts, is not
-// timed, but the smallest in shared memory, as shape 8 is for even ones
+// every tile holds 64 to 512 patterns; shape 13, for odd counts, is the smallest
+// in shared memory, as shape 8 is for even ones; the last two are for 6 categories
 constexpr Shape4 kShapes4[] = {{128, 1, true, 1, 0, 1, false},  {128, 2, true, 1, 0, 1, false},
                                {256, 1, true, 1, 0, 1, false},  {256, 1, false, 1, 0, 1, false},
                                {128, 2, false, 1, 0, 1, false}, {512, 1, false, 1, 0, 1, false},
@@ -779,9 +788,20 @@ constexpr Shape4 kShapes4[] = {{128, 1, true, 1, 0, 1, false},  {128, 2, true, 1
                                {128, 1, false, 2, 0, 2, false}, {256, 2, true, 2, 0, 4, false},
                                {128, 2, true, 2, 0, 4, false},  {128, 4, true, 2, 0, 1, true},
                                {128, 2, true, 1, 4, 1, true},
-                               {128, 1, false, 1, 0, 1, false}};
-constexpr int kNumShapes4 = 13;   // timed
-constexpr int kSmallOdd4 = 13, kSmallEven4 = 8;
+                               {128, 1, false, 1, 0, 1, false},
+                               {128, 1, false, 2, 0, 6, false}, {256, 1, false, 2, 0, 6, false}};
+constexpr int kNumShapes4 = 16, kFirstShapes4 = 13;
+constexpr int kSmallOdd4 = 13, kSmallEven4 = 8, kShared4 = 14;
+// Shapes 14 and 15 are 8 and 7 with two lanes of two pairs for 6 categories, the
+// middle pair formed by both, where those take one lane of three.  They run in
+// their place for trees whose decks are more than 3/2 of a block's shared memory
+// (from some 450 taxa), of which clade tables leave too many to stage: a
+// chain of loads through L1 then bounds every node, and a lane's is a third
+// shorter (us an evaluation, one lane and two: 500 taxa x 3,000 sites 442 and 354,
+// 900 x 500 918 and 709).  Smaller trees are bound by issue, and the pair formed
+// twice costs more than it gives (420 x 2,000 285 and 328, 300 x 3,000 115 and 121,
+// 64 x 150,000 105 and 111).
+bool sharedPair4(int nCat, int nNodes) { return nCat == 6 && nNodes * deckFloats(4, nCat) * 4 > PRUNE_SMEM_MAX / 2 * 3; }
 
 // Where a caller may ask for a shape: (threads, tile, decks staged) as the
 // numbers were first given out, 16 floats a deck and category.  The forms above
@@ -793,15 +813,15 @@ struct First4 {
     int tp, tile;
     bool sdeck;
 };
-constexpr First4 kFirst4[kNumShapes4] = {{128, 128, true},  {128, 256, true},  {256, 256, true}, {256, 256, false},
+constexpr First4 kFirst4[kFirstShapes4] = {{128, 128, true},  {128, 256, true},  {256, 256, true}, {256, 256, false},
                                          {128, 256, false}, {512, 512, false}, {256, 64, false}, {256, 128, false},
                                          {128, 64, false},  {256, 64, true},   {512, 128, false}, {256, 256, true},
                                          {128, 256, true}};
 
 constexpr int lanes4(int nCat, int shape)
 {
-    const int g = kShapes4[shape].g, pairs = (nCat + 1) / 2;
-    return (nCat % 2 == 0 && pairs % g == 0) ? g : 1;
+    const int g = kShapes4[shape].g;
+    return (nCat % 2 == 0 && nCat / 2 % g == 0) || shape >= kShared4 ? g : 1;
 }
 constexpr int threads4(int nCat, int shape) { return kShapes4[shape].tp / kShapes4[shape].g * lanes4(nCat, shape); }
 
@@ -843,6 +863,8 @@ int launchCat4(const PruneJob *dJobs, const BlockDesc *dBlocks, int nTiles, int 
     case 10: if constexpr (NC % 4 == 0) return launchShape4<NC, 10>(dJobs, dBlocks, nTiles, smemBytes, s, nTilesDev, early); break;
     case 11: if constexpr (NC == 3 || NC == 4) return launchShape4<NC, 11>(dJobs, dBlocks, nTiles, smemBytes, s, nTilesDev, early); break;
     case 12: if constexpr (NC == 3 || NC == 4) return launchShape4<NC, 12>(dJobs, dBlocks, nTiles, smemBytes, s, nTilesDev, early); break;
+    case kShared4: if constexpr (NC == 6) return launchShape4<NC, kShared4>(dJobs, dBlocks, nTiles, smemBytes, s, nTilesDev, early); break;
+    case kShared4 + 1: if constexpr (NC == 6) return launchShape4<NC, kShared4 + 1>(dJobs, dBlocks, nTiles, smemBytes, s, nTilesDev, early); break;
     case kSmallOdd4: if constexpr (NC % 2 == 1) return launchShape4<NC, kSmallOdd4>(dJobs, dBlocks, nTiles, smemBytes, s, nTilesDev, early); break;
 #undef P4G_SH
     default: break;
@@ -857,6 +879,7 @@ int prune4NumShapes() { return kNumShapes4; }
 int prune4ShapeValid(int nCat, int shape)
 {
     if (shape == kSmallOdd4) return nCat % 2;
+    if (shape >= kShared4 && shape < kNumShapes4) return nCat == 6;
     if (shape < 0 || shape >= kNumShapes4) return 0;
     if (kShapes4[shape].only34) return nCat == 3 || nCat == 4;
     return nCat % kShapes4[shape].div == 0;
@@ -868,7 +891,22 @@ int prune4KernelExists(int nCat, int shape)
 }
 
 int prune4Tile(int nCat, int shape) { return threads4(nCat, shape) / lanes4(nCat, shape) * kShapes4[shape].ppt; }
-int prune4Smallest(int nCat) { return nCat % 2 ? kSmallOdd4 : kSmallEven4; }
+int prune4ShapeTimed(int nCat, int shape, int nNodes)
+{
+    if (!prune4ShapeValid(nCat, shape) || shape == kSmallOdd4) return 0;
+    const bool two = shape >= kShared4, one = shape == 7 || shape == 8;
+    return nCat != 6 || !(two || one) || two == sharedPair4(nCat, nNodes);
+}
+
+int prune4Smallest(int nCat, int nNodes)
+{
+    return nCat % 2 ? kSmallOdd4 : sharedPair4(nCat, nNodes) ? kShared4 : kSmallEven4;
+}
+
+// Clade tables' first shape: the combinations are few, so lane groups of 2 split the
+// categories and the tables spread over more blocks; P decks are read through L1 (a
+// clade touches few of them).
+int prune4CladeShape(int nCat, int nNodes) { return nCat % 2 ? 3 : prune4Smallest(nCat, nNodes); }
 
 int prune4SmemBytes(int nCat, int nProg, int nDecks, int nRows, int nSlots, int shape, int nClade)
 {
@@ -878,7 +916,7 @@ int prune4SmemBytes(int nCat, int nProg, int nDecks, int nRows, int nSlots, int 
 
 int prune4FirstBytes(int nCat, int nProg, int nDecks, int nRows, int nSlots, int shape, int nClade)
 {
-    if (shape >= kNumShapes4) return INT_MAX;
+    if (shape >= kFirstShapes4) return INT_MAX;
     const First4 &F = kFirst4[shape];
     return layout4(nProg, 0, nRows, nCat, F.tp, F.tile, nSlots, false, nClade).total + (F.sdeck ? nDecks * nCat * 64 : 0);
 }
