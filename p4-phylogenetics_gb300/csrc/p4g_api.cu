@@ -2866,13 +2866,15 @@ static int batchPack(Batch *b, bool &reshape)
         for (size_t gi = 0; gi < b->groups.size(); gi++) {   // every tree tiled like the batch's launch
             PruneGroup &tg = dv.groups[gi];
             if (tg.shape == b->groups[gi].shape) continue;
-            RET(waitImage(t));
-            tg.shape = b->groups[gi].shape;
-            tg.smem = pruneSmemBytes(tg.dim, tg.nCat, dv.nProg, t->nNodes, t->data->nTax, dv.nSlots, tg.shape,
-                                     dv.nClade, dv.nDeck, dv.nRow);
-            if (tg.smem > 227 * 1024)
+            const int shape = b->groups[gi].shape;
+            const int smem = pruneSmemBytes(tg.dim, tg.nCat, dv.nProg, t->nNodes, t->data->nTax, dv.nSlots, shape,
+                                            dv.nClade, dv.nDeck, dv.nRow);
+            if (smem > PRUNE_SMEM_MAX)   // the tree keeps the shape that its tiles are laid out for
                 return setError(P4G_EUNSUPPORTED, "batch: tree %d does not fit the batch's tile shape %d",
-                                (int)ti, tg.shape);
+                                (int)ti, shape);
+            RET(waitImage(t));
+            tg.shape = shape;
+            tg.smem = smem;
             RET(layoutBlocks(t));
         }
         int nDesc, tG, tE, tD, md;
